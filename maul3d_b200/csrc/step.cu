@@ -38,6 +38,7 @@
 #include "m3_solver.cuh"
 #include "m3_joints.cuh"
 #include "m3_tree.h"
+#include "m3_treewalk.cuh"
 #include "m3_ops.h"
 #include "m3_toi.cuh"
 
@@ -162,6 +163,7 @@ struct m3Scratch
     int32_t* treeMoveShape; // M3_TREE_LAG x shapeCap: a step's moves (shapes, ascending)
     m3Aabb* treeMoveBox;   // M3_TREE_LAG x shapeCap: the fat bounds they are inserted with
     uint32_t* gridBar;     // 4 words: the wide kernels' grid barrier (count, generation, error)
+    int32_t* treeState;    // M3_TREE_STATE_WORDS: the tree replay's mode and unbalanced nodes
     int32_t* staticList;   // per shape: static-target flags, then their scan
     int32_t* targetList;   // the continuous phase's static targets, ascending
     int2* jointBodies;     // per joint row: its two bodies (the level walk's compact input)
@@ -246,7 +248,13 @@ static __host__ __device__ inline int64_t ScratchCarve(m3Scratch* s, uint8_t* ba
     M3_CARVE(leafBox, m3Aabb, shapeCap)
     M3_CARVE(hasLeaf, int32_t, shapeCap)
     M3_CARVE(treeMoveCount, int32_t, M3_TREE_LAG)
-    M3_CARVE(gridBar, uint32_t, 4)
+    // The barrier's words and the tree replay's share one aligned piece
+    // (the second need no room of their own).
+    M3_CARVE(gridBar, uint32_t, 4 + M3_TREE_STATE_WORDS)
+    if (s)
+    {
+        s->treeState = (int32_t*)s->gridBar + 4;
+    }
     M3_CARVE(staticList, int32_t, shapeCap + 1)
     M3_CARVE(targetList, int32_t, shapeCap)
     M3_CARVE(jointBodies, int2, jointCap)
@@ -422,14 +430,28 @@ __device__ __forceinline__ uint64_t OrderKey(double x)
 // The broadphase tree's leaves as the broadphase reads them: each
 // shape's leaf bounds, copied out of the tree once per batch; the
 // broadphase keeps the copy current as it moves leaves, so its
-// containment tests never wait for the tree kernel.
+// containment tests never wait for the tree kernel.  The same pass sets
+// up the tree's replay (m3_treewalk.cuh): which nodes are out of balance,
+// and whether its walks may stop early at all.
 __global__ void __launch_bounds__(M3_BLOCK) m3LeafBoxKernel(const m3WorldView* views,
                                                            int32_t count)
 {
     const m3WorldView& w = views[blockIdx.x];
     const m3WorldScalars* sc = w.sc;
+    __shared__ int32_t s_unbalanced;
+    __shared__ int32_t s_full;
     m3Scratch s;
     ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    if (threadIdx.x == 0)
+    {
+        s_unbalanced = 0;
+        s_full = 0;
+    }
+    if (threadIdx.x < M3_TREE_STATE_WORDS)
+    {
+        s.treeState[threadIdx.x] = M3_TREE_NULL;
+    }
+    __syncthreads();
     const int32_t shapeMax = sc->shapeMax;
     for (int32_t i = threadIdx.x; i < shapeMax; i += blockDim.x)
     {
@@ -447,64 +469,148 @@ __global__ void __launch_bounds__(M3_BLOCK) m3LeafBoxKernel(const m3WorldView* v
             s.leafBox[i] = b;
         }
     }
-}
-
-// Broadphase tree refresh, second half (broad_phase.c:516-538): one warp
-// per world replays one step's moves in ascending shape order, each a
-// leaf removal and the insertion of its fat bounds; the warp's lanes
-// prefetch the world's nodes into L2, lane 0 walks.  (One lane per world,
-// 32 worlds to a warp, measured several times slower: the worlds' walks
-// diverge and their dependent loads serialise.)  The tree is state only a
-// snapshot reads, so this runs on its own stream beside the following
-// steps, each world up to M3_TREE_LAG steps behind (the move lists sit in
-// a ring of that depth).
-// One step's leaf moves of one world, replayed by lane 0 (the lanes
-// have prefetched the world's nodes).
-__device__ void m3ReplayTreeStep(const m3WorldView& w, const m3Scratch& s, int32_t slot,
-                                 int32_t moves)
-{
-    m3WorldScalars* sc = w.sc;
-    const m3TreeRef tree = m3WorldTree(w);
-    // Observer only: leaf moves replayed, in the phase counters' spare
-    // slot (a count, not cycles).
-    sc->phase[15] += (uint64_t)moves;
-    const m3TreeArrayStore store{w.treeNodes};
-    const int32_t* shapes = s.treeMoveShape + (int64_t)slot * sc->shapeCap;
-    const m3Aabb* boxes = s.treeMoveBox + (int64_t)slot * sc->shapeCap;
-    const int32_t shapeMax = sc->shapeMax;
-    const int32_t nodeCap = 2 * sc->shapeCap;
-    for (int32_t m = 0; m < moves; ++m)
+    if (sc->treeTracked == 0)
     {
-        const int32_t shape = shapes[m];
-        const m3Aabb box = boxes[m];
-        const int32_t old = shape >= 0 && shape < shapeMax ? w.proxyId[shape] : M3_TREE_NULL;
-        if (old == M3_TREE_NULL || old < 0 || old >= nodeCap)
+        return;
+    }
+    const int32_t nodeCap = 2 * sc->shapeCap;
+    for (int32_t i = threadIdx.x; i < nodeCap; i += blockDim.x)
+    {
+        const m3TreeNode n = w.treeNodes[i];
+        if (n.height < 0)
         {
-            // Only shapes with a leaf are ever recorded as moves.
-            atomicExch(&sc->status, M3GPU_ERR_INVALID);
-            sc->statusDetail = 6001;
-            return;
+            continue; // free
         }
-        m3TreeRemove(tree, store, old);
-        const int32_t leaf = m3TreeInsert(tree, store, box.lo, box.hi, shape);
-        w.proxyId[shape] = leaf;
-        if (leaf == M3_TREE_NULL)
+        bool plain = true;
+        if (n.height == 0)
         {
-            // The reference's pair update refuses with m3_errorCapacity.
-            atomicExch(&sc->status, M3GPU_ERR_CAPACITY);
-            return;
+            plain = m3TreePlainBox(n.lo, n.hi);
+        }
+        else
+        {
+            const m3TreeNode a = w.treeNodes[n.child1];
+            const m3TreeNode b = w.treeNodes[n.child2];
+            double lo[3];
+            double hi[3];
+            m3TreeUnion(a.lo, a.hi, b.lo, b.hi, lo, hi);
+            for (int32_t k = 0; k < 3; ++k)
+            {
+                plain = plain &&
+                        __double_as_longlong(lo[k]) == __double_as_longlong(n.lo[k]) &&
+                        __double_as_longlong(hi[k]) == __double_as_longlong(n.hi[k]);
+            }
+            plain = plain && n.height == 1 + m3TreeMaxI(a.height, b.height);
+            const int32_t tilt = a.height - b.height;
+            if (tilt > 1 || tilt < -1)
+            {
+                const int32_t at = atomicAdd(&s_unbalanced, 1);
+                if (at < M3_TREE_STATE_WORDS - 1)
+                {
+                    s.treeState[1 + at] = i;
+                }
+                else
+                {
+                    plain = false;
+                }
+            }
+        }
+        if (!plain)
+        {
+            s_full = 1;
         }
     }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        s.treeState[0] = s_full != 0 ? M3_TREE_FULL : M3_TREE_TRACKED;
+    }
+}
+
+// Broadphase tree refresh, second half (broad_phase.c:516-538): one block
+// of two warps per world replays its recorded steps' moves in order, each
+// a leaf removal and the insertion of its fat bounds (m3_treewalk.cuh).
+// (One lane per world, 32 worlds to a warp, measured several times
+// slower: the worlds' walks diverge and their dependent loads serialise.)
+// The first warp walks, the second stages the next 32 moves in shared
+// memory meanwhile.  (The second warp walking ahead of those moves to warm
+// L1 measured no gain for one world, whose walks hit L1 99 % of the time,
+// and twice the time for a large batch.)
+// The tree is state only a snapshot reads, so this runs on its own stream
+// beside the following steps, each world up to M3_TREE_LAG steps behind
+// (the move lists sit in a ring of that depth).
+#define M3_TREE_CHUNK 32
+#define M3_TREE_THREADS 64
+struct m3TreeChunk
+{
+    m3Aabb box[M3_TREE_CHUNK];
+    int32_t shape[M3_TREE_CHUNK];
+    int32_t leaf[M3_TREE_CHUNK];
+    int32_t count;
+    int32_t plain; // the walks may stop early with every box
+};
+
+// Where a replay stands in its steps' move lists.
+struct m3TreeCursor
+{
+    int32_t step; // of `steps` recorded steps
+    int32_t move; // within the step
+};
+
+// Stages the chunk at the cursor (one warp) and moves the cursor past it;
+// an empty chunk says that every step is done.
+__device__ void m3StageTreeChunk(const m3WorldView& w, const m3Scratch& s, int32_t tail,
+                                 int32_t steps, int32_t treeLag, m3TreeCursor* at,
+                                 m3TreeChunk* chunk, int32_t lane)
+{
+    const m3WorldScalars* sc = w.sc;
+    const int32_t shapeMax = sc->shapeMax;
+    int32_t n = 0;
+    int32_t slot = 0;
+    while (at->step < steps)
+    {
+        slot = (int32_t)((uint32_t)(tail + at->step) % (uint32_t)treeLag);
+        // A move count above the shape slots cannot come from this
+        // world's broadphase.
+        const int32_t moves = s.treeMoveCount[slot];
+        if (moves > at->move && moves <= shapeMax)
+        {
+            n = moves - at->move < M3_TREE_CHUNK ? moves - at->move : M3_TREE_CHUNK;
+            break;
+        }
+        at->step += 1;
+        at->move = 0;
+    }
+    bool plain = true;
+    if (lane < n)
+    {
+        const int64_t m = (int64_t)slot * sc->shapeCap + at->move + lane;
+        const int32_t shape = s.treeMoveShape[m];
+        const m3Aabb box = s.treeMoveBox[m];
+        plain = m3TreePlainBox(box.lo, box.hi);
+        int32_t leaf = shape >= 0 && shape < shapeMax ? w.proxyId[shape] : M3_TREE_NULL;
+        leaf = leaf >= 0 && leaf < 2 * sc->shapeCap ? leaf : M3_TREE_NULL;
+        chunk->box[lane] = box;
+        chunk->shape[lane] = shape;
+        chunk->leaf[lane] = leaf;
+    }
+    plain = __all_sync(M3_FULL_WARP, plain);
+    if (lane == 0)
+    {
+        chunk->count = n;
+        chunk->plain = plain ? 1 : 0;
+    }
+    at->move += n;
 }
 
 // The replay of each world's oldest `steps[world]` recorded steps (the
 // world's index in `views`), in the order the broadphase recorded them.
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(M3_TREE_THREADS)
     m3TreeKernel(const m3WorldView* views, const int32_t* order, int32_t count, int32_t treeLag,
                  const int32_t* steps)
 {
     const int32_t k = blockIdx.x;
-    const int32_t lane = (int32_t)threadIdx.x;
+    const int32_t lane = (int32_t)threadIdx.x & 31;
+    const bool walker = threadIdx.x < 32;
     if (k >= count)
     {
         return;
@@ -517,24 +623,28 @@ __global__ void __launch_bounds__(32)
     {
         return;
     }
+    __shared__ m3TreeChunk chunks[2];
+    __shared__ int32_t s_stop;
     m3Scratch s;
     ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap, treeLag);
     const int32_t tail = sc->treeTail;
-    __syncwarp();
-    if (lane == 0)
+    const bool refused = sc->status != 0;
+    __syncthreads();
+    if (threadIdx.x == 0)
     {
         sc->treeTail = tail + n;
+        s_stop = 0;
     }
     // A refused world's tree is not kept (its state is unspecified after
     // a refusal).
-    if (sc->status != 0)
+    if (refused)
     {
         return;
     }
-    // The walk below is a chain of dependent loads: bring the world's
-    // nodes into L2 first, one bulk prefetch per 64 KiB piece (the array
-    // is 256-byte aligned and 144 bytes a shape, so every piece is a
-    // multiple of 16 bytes).
+    // Bring the world's nodes into L2 first, one bulk prefetch per 64 KiB
+    // piece (the array is 256-byte aligned and 144 bytes a shape, so every
+    // piece is a multiple of 16 bytes).
+    if (walker)
     {
         const int64_t bytes = (int64_t)sizeof(m3TreeNode) * 2 * sc->shapeCap;
         const uint8_t* base = (const uint8_t*)w.treeNodes;
@@ -546,24 +656,72 @@ __global__ void __launch_bounds__(32)
                          : "memory");
         }
     }
-    if (lane != 0)
+    m3TreeWarp tree;
+    tree.nodes = w.treeNodes;
+    tree.capacity = 2 * sc->shapeCap;
+    tree.root = sc->treeRoot;
+    tree.lane = lane;
+    tree.bound = lane < 5 ? lane : 5;
+    tree.unbalanced = s.treeState[1 + lane];
+    tree.tracked = s.treeState[0] == M3_TREE_TRACKED;
+    m3TreeCursor at = {0, 0};
+    if (!walker)
+    {
+        m3StageTreeChunk(w, s, tail, n, treeLag, &at, &chunks[0], lane);
+    }
+    __syncthreads();
+    int32_t total = 0;
+    for (int32_t c = 0;; c ^= 1)
+    {
+        const m3TreeChunk& chunk = chunks[c];
+        const int32_t moves = chunk.count;
+        if (moves == 0 || s_stop != 0)
+        {
+            break;
+        }
+        if (!walker)
+        {
+            m3StageTreeChunk(w, s, tail, n, treeLag, &at, &chunks[c ^ 1], lane);
+        }
+        else
+        {
+            tree.tracked = tree.tracked && chunk.plain != 0;
+            int32_t stop = 0;
+            for (int32_t m = 0; m < moves && stop == 0; ++m)
+            {
+                const int32_t leaf = chunk.leaf[m];
+                // Only shapes with a leaf are ever recorded as moves; a
+                // descent without end is a malformed tree (the reference's
+                // pair update refuses with m3_errorCapacity).
+                stop = leaf == M3_TREE_NULL ? M3GPU_ERR_INVALID
+                       : tree.Move(leaf, chunk.shape[m], chunk.box[m].lo) ? 0
+                                                                          : M3GPU_ERR_CAPACITY;
+            }
+            if (lane == 0 && stop != 0)
+            {
+                atomicExch(&sc->status, stop);
+                if (stop == M3GPU_ERR_INVALID)
+                {
+                    sc->statusDetail = 6001;
+                }
+                s_stop = 1;
+            }
+            total += moves;
+        }
+        __syncthreads();
+    }
+    if (!walker)
     {
         return;
     }
-    for (int32_t i = 0; i < n; ++i)
+    s.treeState[1 + lane] = tree.unbalanced;
+    if (lane == 0)
     {
-        const int32_t slot = (int32_t)((uint32_t)(tail + i) % (uint32_t)treeLag);
-        const int32_t moves = s.treeMoveCount[slot];
-        // A move count above the shape slots cannot come from this
-        // world's broadphase.
-        if (moves > 0 && moves <= sc->shapeMax)
-        {
-            m3ReplayTreeStep(w, s, slot, moves);
-        }
-        if (sc->status != 0)
-        {
-            return;
-        }
+        s.treeState[0] = tree.tracked ? M3_TREE_TRACKED : M3_TREE_FULL;
+        sc->treeRoot = tree.root;
+        // Observer only: leaf moves replayed, in the phase counters' spare
+        // slot (a count, not cycles).
+        sc->phase[15] += (uint64_t)total;
     }
 }
 
@@ -5168,7 +5326,7 @@ static void LaunchTreeReplay(m3TreeTable* table, m3HostWorld** worlds, int32_t c
     }
     cudaMemcpyAsync(table->steps, table->hostSteps, sizeof(int32_t) * (size_t)count,
                     cudaMemcpyHostToDevice, stream);
-    m3TreeKernel<<<count, 32, 0, stream>>>(table->views, table->order, count, M3_TREE_LAG,
+    m3TreeKernel<<<count, M3_TREE_THREADS, 0, stream>>>(table->views, table->order, count, M3_TREE_LAG,
                                            table->steps);
     const uint64_t q = RecordTreeLaunch(stream);
     table->lastSeq = q;
@@ -5246,7 +5404,7 @@ void m3gpuWaitTree(m3HostWorld* w)
         const int32_t table[2] = {0, w->treeUnlaunched};
         cudaMemcpy(s_oneView, &view, sizeof(view), cudaMemcpyHostToDevice);
         cudaMemcpy(s_oneOrder, table, sizeof(table), cudaMemcpyHostToDevice);
-        m3TreeKernel<<<1, 32>>>(s_oneView, s_oneOrder, 1, M3_TREE_LAG, s_oneSteps);
+        m3TreeKernel<<<1, M3_TREE_THREADS>>>(s_oneView, s_oneOrder, 1, M3_TREE_LAG, s_oneSteps);
         s_launches += 1;
     }
     w->treeCount = 0;
@@ -5752,7 +5910,7 @@ extern "C" int32_t m3gpu_step_world_noalloc(m3WorldId worldId, float dt, int32_t
     w->leafBoxValid = false;
     m3LeafBoxKernel<<<1, M3_BLOCK>>>(sym.view, 1);
     m3BroadKernel<M3_BLOCK, 1><<<1, M3_BLOCK>>>(sym.view, order, 1, 1);
-    m3TreeKernel<<<1, 32>>>(sym.view, order, 1, 1, sym.table + 3);
+    m3TreeKernel<<<1, M3_TREE_THREADS>>>(sym.view, order, 1, 1, sym.table + 3);
     m3PairOffsetsKernel<<<1, M3_BLOCK>>>(sym.view, 1, offsets);
     m3NarrowKernel<<<148, 128>>>(sym.view, offsets, 1);
     LaunchSolve(sym.view, order, 1, dt, substeps, cacheBytes, nullptr);
