@@ -64,6 +64,14 @@
 #define M3_WW_PART 32       // M3_WIDE_MAX_BLOCKS + 1 words: the grid scan's block totals
 #define M3_WW_BLOCKCOLOR (M3_WW_PART + M3_WIDE_MAX_BLOCKS + 1)
 #define M3_WW_WORDS (M3_WW_BLOCKCOLOR + M3_WIDE_MAX_BLOCKS * (M3_GRAPH_COLORS + 1))
+// A wide world's broadphase words between its kernels.
+#define M3_BS_PLANES 0
+#define M3_BS_SWEEP 1
+#define M3_BS_PAIRS 2
+#define M3_BS_SLOT 3
+#define M3_BS_LONG 4
+#define M3_BS_PLANE0 8
+#define M3_BS_WORDS (M3_BS_PLANE0 + M3_MAX_PLANES)
 // Colouring: the marker of a constraint not coloured yet, and the
 // parallel rounds before the serial finish (one block per world; a wide
 // world's grid affords many more rounds).
@@ -167,7 +175,7 @@ struct m3Scratch
     int32_t* staticList;   // per shape: static-target flags, then their scan
     int32_t* targetList;   // the continuous phase's static targets, ascending
     int2* jointBodies;     // per joint row: its two bodies (the level walk's compact input)
-    int32_t* broadState;   // 20 words: a wide world's broadphase between its kernels
+    int32_t* broadState;   // M3_BS_WORDS: a wide world's broadphase between its kernels
     int32_t* wideWork;     // the wide prepare kernel's grid-shared words (M3_WW_*)
     int32_t* jointAdj;     // 2 per joint row: rows by body (the wide joint levels)
     int2* jointPrev;       // per joint row: the previous row on each of its bodies
@@ -258,7 +266,7 @@ static __host__ __device__ inline int64_t ScratchCarve(m3Scratch* s, uint8_t* ba
     M3_CARVE(staticList, int32_t, shapeCap + 1)
     M3_CARVE(targetList, int32_t, shapeCap)
     M3_CARVE(jointBodies, int2, jointCap)
-    M3_CARVE(broadState, int32_t, 4 + M3_MAX_PLANES)
+    M3_CARVE(broadState, int32_t, M3_BS_WORDS)
     M3_CARVE(wideWork, int32_t, M3_WW_WORDS)
     M3_CARVE(jointAdj, int32_t, 2 * (int64_t)jointCap)
     M3_CARVE(jointPrev, int2, jointCap)
@@ -419,13 +427,64 @@ __device__ bool PairAllowed(const m3WorldView& w, int32_t i, int32_t j)
 // key order (broad_phase.c:632-637) without a global sort.
 // ---------------------------------------------------------------------
 
-// Total order on doubles as unsigned integers (negative values flipped).
-__device__ __forceinline__ uint64_t OrderKey(double x)
+// The sweep's sort element of a shape: its x lower bound rounded down to
+// a float, as an unsigned integer of the same order, above its index.
+// The sweep compares floats rounded outward, which keep every overlap of
+// the doubles, and the doubles decide what it finds; so the order of equal
+// floats is free, and a 64-bit element sorts in half the steps of a
+// 64-bit key with an index beside it.
+__device__ __forceinline__ uint64_t SweepKey(double x, int32_t shape)
 {
-    uint64_t b = (uint64_t)__double_as_longlong(x);
-    return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+    const uint32_t b = (uint32_t)__float_as_int(__double2float_rd(x));
+    const uint32_t k = (b >> 31) != 0 ? ~b : b | 0x80000000u;
+    return (uint64_t)k << 32 | (uint32_t)shape;
+}
+#define M3_SWEEP_NONE (~0ull)
+
+// The sorted shapes' boxes as the sweep reads them, rounded outward, one
+// array per bound (the threads of a warp read neighbouring positions).
+// They lie in the contact rows' memory, which the step fills later.
+struct m3SweepBoxes
+{
+    float* at;
+    int32_t stride;
+};
+
+__device__ __forceinline__ m3SweepBoxes SweepBoxes(const m3Scratch& s, int32_t shapeCap)
+{
+    m3SweepBoxes b;
+    b.at = s.rows.ro;
+    b.stride = (int32_t)m3AlignUp(shapeCap, 32);
+    return b;
 }
 
+// The candidates of a per-world sweep (positions p < q whose float boxes
+// overlap), behind the boxes: at most this many a shape slot.
+#define M3_SWEEP_CANDIDATES 64
+__device__ __forceinline__ int2* SweepCandidates(const m3Scratch& s, int32_t shapeCap)
+{
+    const m3SweepBoxes b = SweepBoxes(s, shapeCap);
+    return (int2*)(b.at + 6 * (int64_t)b.stride);
+}
+
+// A second array of sort elements behind the boxes (a wide world's).
+__device__ __forceinline__ uint64_t* SweepSpare(const m3Scratch& s, int32_t shapeCap)
+{
+    const m3SweepBoxes b = SweepBoxes(s, shapeCap);
+    return (uint64_t*)(b.at + 6 * (int64_t)b.stride);
+}
+
+__device__ __forceinline__ void PutSweepBox(const m3Scratch& s, const m3SweepBoxes& boxes,
+                                            int32_t p, int32_t shape)
+{
+    const m3Aabb& box = s.aabb[shape];
+    s.sortIdx[p] = shape;
+    for (int32_t k = 0; k < 3; ++k)
+    {
+        boxes.at[2 * k * (int64_t)boxes.stride + p] = __double2float_rd(box.lo[k]);
+        boxes.at[(2 * k + 1) * (int64_t)boxes.stride + p] = __double2float_ru(box.hi[k]);
+    }
+}
 
 // The broadphase tree's leaves as the broadphase reads them: each
 // shape's leaf bounds, copied out of the tree once per batch; the
@@ -725,30 +784,127 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
     }
 }
 
-// Visit every non-plane pair (a < b) whose fresh bounds overlap and that
-// the filter allows, from the sweep position `p` of the sorted order.
-template <typename F>
-__device__ __forceinline__ void SweepFrom(const m3WorldView& w, const m3Scratch& s, int32_t p,
-                                          int32_t n, F&& visit)
+// One sorted position's box, and its test against another's.
+struct m3SweepBox
 {
-    const int32_t a = s.sortIdx[p];
-    const m3Aabb boxA = s.aabb[a];
-    for (int32_t q = p + 1; q < n; ++q)
+    float lo[3];
+    float hi[3];
+};
+
+__device__ __forceinline__ m3SweepBox GetSweepBox(const m3SweepBoxes& boxes, int32_t p)
+{
+    m3SweepBox b;
+    for (int32_t k = 0; k < 3; ++k)
     {
-        const int32_t b = s.sortIdx[q];
-        const m3Aabb& boxB = s.aabb[b];
-        if (!(boxB.lo[0] <= boxA.hi[0]))
+        b.lo[k] = boxes.at[2 * k * (int64_t)boxes.stride + p];
+        b.hi[k] = boxes.at[(2 * k + 1) * (int64_t)boxes.stride + p];
+    }
+    return b;
+}
+
+// Position q against an earlier position's box: -1 when q and everything
+// behind it starts beyond the box, 1 when the float boxes overlap.
+__device__ __forceinline__ int32_t SweepTest(const m3SweepBoxes& boxes, const m3SweepBox& boxA,
+                                             int32_t q)
+{
+    const float* at = boxes.at + q;
+    const int64_t stride = boxes.stride;
+    if (!(at[0] <= boxA.hi[0]))
+    {
+        return -1;
+    }
+    return at[2 * stride] <= boxA.hi[1] && boxA.lo[1] <= at[3 * stride] &&
+                   at[4 * stride] <= boxA.hi[2] && boxA.lo[2] <= at[5 * stride]
+               ? 1
+               : 0;
+}
+
+// The first position behind p that starts beyond the box (the floats are
+// sorted, NaNs last).
+__device__ __forceinline__ int32_t SweepEnd(const m3SweepBoxes& boxes, const m3SweepBox& boxA,
+                                            int32_t p, int32_t n)
+{
+    int32_t lo = p + 1;
+    int32_t hi = n;
+    while (lo < hi)
+    {
+        const int32_t mid = (lo + hi) >> 1;
+        if (boxes.at[mid] <= boxA.hi[0])
         {
-            break;
+            lo = mid + 1;
         }
-        if (Overlap(boxA, boxB))
+        else
         {
-            int32_t lo = a < b ? a : b;
-            int32_t hi = a < b ? b : a;
-            if (PairAllowed(w, lo, hi))
+            hi = mid;
+        }
+    }
+    return lo;
+}
+
+// Whether position q (before the box's sweep end) overlaps the box in y
+// and z.
+__device__ __forceinline__ bool SweepAcross(const m3SweepBoxes& boxes, const m3SweepBox& boxA,
+                                            int32_t q)
+{
+    const float* at = boxes.at + q;
+    const int64_t stride = boxes.stride;
+    const float loY = at[2 * stride];
+    const float hiY = at[3 * stride];
+    const float loZ = at[4 * stride];
+    const float hiZ = at[5 * stride];
+    return (loY <= boxA.hi[1]) & (boxA.lo[1] <= hiY) & (loZ <= boxA.hi[2]) & (boxA.lo[2] <= hiZ);
+}
+
+// A candidate: visits the pair of shapes a and b (smaller index first) when
+// the fresh bounds overlap and the filter allows it.
+template <typename F>
+__device__ __forceinline__ void SweepVisit(const m3WorldView& w, const m3Scratch& s, int32_t a,
+                                           int32_t b, F&& visit)
+{
+    if (Overlap(s.aabb[a], s.aabb[b]))
+    {
+        const int32_t lo = a < b ? a : b;
+        const int32_t hi = a < b ? b : a;
+        if (PairAllowed(w, lo, hi))
+        {
+            visit(lo, hi);
+        }
+    }
+}
+
+template <typename F>
+__device__ __forceinline__ bool SweepPair(const m3WorldView& w, const m3Scratch& s,
+                                          const m3SweepBoxes& boxes, int32_t a,
+                                          const m3SweepBox& boxA, int32_t q, F&& visit)
+{
+    const int32_t hit = SweepTest(boxes, boxA, q);
+    if (hit > 0)
+    {
+        SweepVisit(w, s, a, s.sortIdx[q], visit);
+    }
+    return hit >= 0;
+}
+
+// Sorts `count` (a power of two) elements in place, in shared or global
+// memory; every thread of the block takes part.
+template <int NT> __device__ __forceinline__ void BlockSort(uint64_t* a, int32_t count)
+{
+    for (int32_t k = 2; k <= count; k <<= 1)
+    {
+        for (int32_t j = k >> 1; j > 0; j >>= 1)
+        {
+            for (int32_t t = threadIdx.x; t < count / 2; t += NT)
             {
-                visit(lo, hi);
+                const int32_t i = 2 * t - (t & (j - 1));
+                const uint64_t x = a[i];
+                const uint64_t y = a[i + j];
+                if ((x > y) == ((i & k) == 0))
+                {
+                    a[i] = y;
+                    a[i + j] = x;
+                }
             }
+            __syncthreads();
         }
     }
 }
@@ -758,20 +914,28 @@ __device__ __forceinline__ void SweepFrom(const m3WorldView& w, const m3Scratch&
 // thread).
 #define M3_LONG_ROW 64
 #define M3_LONG_ROWS 16
+// A long row of c keys is ranked (c x c comparisons) up to this many times
+// the shape slots' count of them, and beyond that its partners are flagged
+// and counted over the slots (a heightfield under 7,001 bodies ranked its
+// row in 1.6 ms a step).
+#define M3_LONG_ROW_FLAGS 16
 
 // PART 0 is the whole broadphase of one world per block.  A wide world
-// splits it around the sweep: PART 1 (bounds, tree moves, sort; one
-// block) leaves the plane list and the sweep count in s.broadState,
-// m3WideSweepKernel counts and records the pairs over the whole grid,
+// runs its bounds, sort and sweep over the whole grid (the m3Wide kernels
+// below, which leave the plane list and the pair count in s.broadState);
 // PART 2 (scan, fill, row order; one block) finishes.
-#define M3_BS_PLANES 0
-#define M3_BS_SWEEP 1
-#define M3_BS_PAIRS 2
-#define M3_BS_PLANE0 4
+//
+// PART 0 sorts in shared memory up to `sortCap` elements (a power of two;
+// larger worlds sort in global memory): a 2048-body world's sort took 83 us
+// in global memory and 24 us here.  A position with more than
+// M3_SWEEP_LONG candidates (a ground, a heightfield: most of the world)
+// leaves them to the whole block.
+#define M3_SWEEP_LONG 256
+#define M3_SWEEP_LONGS 64
 template <int NT, int MIN_BLOCKS, int PART = 0>
 __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldView* views,
                                                           const int32_t* order, int32_t count,
-                                                          int32_t treeLag)
+                                                          int32_t treeLag, int32_t sortCap)
 {
     const int32_t wi = order[blockIdx.x];
     const m3WorldView& w = views[wi];
@@ -779,6 +943,10 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
     m3Scratch s;
     ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap, treeLag);
     const int32_t tid = threadIdx.x;
+    extern __shared__ uint64_t s_sort[];
+    __shared__ int2 s_long[M3_SWEEP_LONGS];
+    __shared__ int32_t s_longSweeps;
+    __shared__ int32_t s_candidates;
     __shared__ int32_t s_status;
     __shared__ int32_t s_planes[M3_MAX_PLANES];
     __shared__ int32_t s_planeCount;
@@ -791,6 +959,8 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
         s_planeCount = 0;
         s_sweepCount = 0;
         s_sweepPairs = 0;
+        s_longSweeps = 0;
+        s_candidates = 0;
         // A world that keeps the tree records one ring slot per step, read
         // back by exactly one tree launch.  No moves are recorded unless
         // this step reaches the containment tests below: the tree kernel
@@ -804,17 +974,16 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
             s.treeMoveCount[slot] = 0;
         }
         s_treeSlot = slot;
-        if (PART == 1)
-        {
-            // The wide kernels of this step start their grid barrier
-            // with no arrivals and no error.
-            s.gridBar[0] = 0;
-            s.gridBar[2] = 0;
-        }
         if (PART == 2 && s_status == 0)
         {
             s_planeCount = s.broadState[M3_BS_PLANES];
             s_sweepPairs = s.broadState[M3_BS_PAIRS];
+            if (s_planeCount > M3_MAX_PLANES)
+            {
+                sc->status = M3GPU_ERR_UNSUPPORTED;
+                sc->statusDetail = 5001;
+                s_status = M3GPU_ERR_UNSUPPORTED;
+            }
             for (int32_t k = 0; k < s_planeCount && k < M3_MAX_PLANES; ++k)
             {
                 s_planes[k] = s.broadState[M3_BS_PLANE0 + k];
@@ -832,7 +1001,14 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
     if (PART != 2)
     {
 
-    // Fresh bounds once per shape; the sweep set and the plane list.
+    // Fresh bounds once per shape; the sweep's elements (in any order) and
+    // the plane list.
+    int32_t pow2 = 1;
+    while (pow2 < shapeMax)
+    {
+        pow2 <<= 1;
+    }
+    uint64_t* elems = pow2 <= sortCap ? s_sort : s.sortKey;
     for (int32_t i = tid; i < shapeMax; i += NT)
     {
         s.rowCount[i] = 0;
@@ -850,9 +1026,10 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
             }
             continue;
         }
-        s.aabb[i] = ShapeBounds(w, i);
+        const m3Aabb box = ShapeBounds(w, i);
+        s.aabb[i] = box;
         int32_t k = atomicAdd(&s_sweepCount, 1);
-        s.sortIdx[k] = i;
+        elems[k] = SweepKey(box.lo[0], i);
     }
     __syncthreads();
     if (s_planeCount > M3_MAX_PLANES)
@@ -911,82 +1088,118 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
     }
     M3_PHASE_MARK(M3_PHASE_BOUNDS)
     const int32_t n = s_sweepCount;
-    int32_t pow2 = 1;
+    pow2 = 1;
     while (pow2 < n)
     {
         pow2 <<= 1;
     }
-    for (int32_t i = tid; i < pow2; i += NT)
+    for (int32_t i = n + tid; i < pow2; i += NT)
     {
-        if (i < n)
-        {
-            s.sortKey[i] = OrderKey(s.aabb[s.sortIdx[i]].lo[0]);
-        }
-        else
-        {
-            s.sortKey[i] = ~0ull;
-            s.sortIdx[i] = 0x7FFFFFFF;
-        }
+        elems[i] = M3_SWEEP_NONE;
     }
     __syncthreads();
-    // Bitonic sort by (x lower bound, shape index).
-    for (int32_t k = 2; k <= pow2; k <<= 1)
+    if (pow2 <= sortCap)
     {
-        for (int32_t j = k >> 1; j > 0; j >>= 1)
-        {
-            for (int32_t i = tid; i < pow2; i += NT)
-            {
-                int32_t ixj = i ^ j;
-                if (ixj > i)
-                {
-                    uint64_t ka = s.sortKey[i];
-                    uint64_t kb = s.sortKey[ixj];
-                    int32_t ia = s.sortIdx[i];
-                    int32_t ib = s.sortIdx[ixj];
-                    bool greater = ka > kb || (ka == kb && ia > ib);
-                    bool ascending = (i & k) == 0;
-                    if (greater == ascending)
-                    {
-                        s.sortKey[i] = kb;
-                        s.sortKey[ixj] = ka;
-                        s.sortIdx[i] = ib;
-                        s.sortIdx[ixj] = ia;
-                    }
-                }
-            }
-            __syncthreads();
-        }
+        BlockSort<NT>(s_sort, pow2);
     }
-
+    else
+    {
+        BlockSort<NT>(s.sortKey, pow2);
+    }
+    const m3SweepBoxes boxes = SweepBoxes(s, sc->shapeCap);
+    for (int32_t p = tid; p < n; p += NT)
+    {
+        PutSweepBox(s, boxes, p, (int32_t)(uint32_t)elems[p]);
+    }
+    __syncthreads();
     M3_PHASE_MARK(M3_PHASE_SORT)
-    if (PART == 1)
-    {
-        if (tid == 0)
-        {
-            s.broadState[M3_BS_PLANES] = s_planeCount;
-            s.broadState[M3_BS_SWEEP] = n;
-            s.broadState[M3_BS_PAIRS] = 0;
-            for (int32_t k = 0; k < s_planeCount; ++k)
-            {
-                s.broadState[M3_BS_PLANE0 + k] = s_planes[k];
-            }
-        }
-        return;
-    }
     // Count every row's pairs; the sweep's pairs are recorded on the way
     // so the fill below need not sweep again.
     const int32_t planeCount = s_planeCount;
     const int32_t pairCap = sc->pairCap;
+    const auto record = [&](int32_t lo, int32_t hi) {
+        atomicAdd(&s.rowCount[lo], 1);
+        const int32_t r = atomicAdd(&s_sweepPairs, 1);
+        if (r < pairCap)
+        {
+            s.sweepPairs[r] = ((uint64_t)(uint32_t)lo << 32) | (uint64_t)(uint32_t)hi;
+        }
+    };
+    // The float sweep lists its candidates; then every thread takes its
+    // share of them through the exact test and the filter, whose dependent
+    // loads would otherwise follow one another in a position's own thread.
+    int2* candidates = SweepCandidates(s, sc->shapeCap);
+    const int32_t candidateCap = M3_SWEEP_CANDIDATES * sc->shapeCap;
+    const auto candidate = [&](int32_t p, int32_t q) {
+        const int32_t k = atomicAdd(&s_candidates, 1);
+        if (k < candidateCap)
+        {
+            candidates[k] = make_int2(s.sortIdx[p], s.sortIdx[q]);
+        }
+        else
+        {
+            SweepVisit(w, s, s.sortIdx[p], s.sortIdx[q], record);
+        }
+    };
     for (int32_t p = tid; p < n; p += NT)
     {
-        SweepFrom(w, s, p, n, [&](int32_t lo, int32_t hi) {
-            atomicAdd(&s.rowCount[lo], 1);
-            const int32_t r = atomicAdd(&s_sweepPairs, 1);
-            if (r < pairCap)
+        const m3SweepBox boxA = GetSweepBox(boxes, p);
+        int32_t end = SweepEnd(boxes, boxA, p, n);
+        if (end - p > M3_SWEEP_LONG)
+        {
+            const int32_t k = atomicAdd(&s_longSweeps, 1);
+            if (k < M3_SWEEP_LONGS)
             {
-                s.sweepPairs[r] = ((uint64_t)(uint32_t)lo << 32) | (uint64_t)(uint32_t)hi;
+                s_long[k] = make_int2(p, end);
+                end = p;
             }
-        });
+        }
+        // Four positions' loads under way at a time.
+        int32_t q = p + 1;
+        for (; q + 3 < end; q += 4)
+        {
+            bool hit[4];
+#pragma unroll
+            for (int32_t k = 0; k < 4; ++k)
+            {
+                hit[k] = SweepAcross(boxes, boxA, q + k);
+            }
+#pragma unroll
+            for (int32_t k = 0; k < 4; ++k)
+            {
+                if (hit[k])
+                {
+                    candidate(p, q + k);
+                }
+            }
+        }
+        for (; q < end; ++q)
+        {
+            if (SweepAcross(boxes, boxA, q))
+            {
+                candidate(p, q);
+            }
+        }
+    }
+    __syncthreads();
+    const int32_t longSweeps = s_longSweeps < M3_SWEEP_LONGS ? s_longSweeps : M3_SWEEP_LONGS;
+    for (int32_t k = 0; k < longSweeps; ++k)
+    {
+        const int2 range = s_long[k];
+        const m3SweepBox boxA = GetSweepBox(boxes, range.x);
+        for (int32_t q = range.x + 1 + tid; q < range.y; q += NT)
+        {
+            if (SweepAcross(boxes, boxA, q))
+            {
+                candidate(range.x, q);
+            }
+        }
+    }
+    __syncthreads();
+    const int32_t listed = s_candidates < candidateCap ? s_candidates : candidateCap;
+    for (int32_t k = tid; k < listed; k += NT)
+    {
+        SweepVisit(w, s, candidates[k].x, candidates[k].y, record);
     }
     for (int32_t i = tid; i < shapeMax; i += NT)
     {
@@ -1136,13 +1349,40 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
         }
     }
     __syncthreads();
-    // The long rows; the sweep's pair list is spent and holds each row's
-    // sorted copy (a row is no longer than the pair capacity).
+    // The long rows; the sweep's pair list is spent and holds each ranked
+    // row's sorted copy (a row is no longer than the pair capacity).
     const int32_t longRows = s_longCount < M3_LONG_ROWS ? s_longCount : M3_LONG_ROWS;
     for (int32_t r = 0; r < longRows; ++r)
     {
-        const int32_t a = s.rowCount[s_longRows[r]];
-        const int32_t c = s.rowFill[s_longRows[r]];
+        const int32_t row = s_longRows[r];
+        const int32_t a = s.rowCount[row];
+        const int32_t c = s.rowFill[row];
+        if ((int64_t)c * c > M3_LONG_ROW_FLAGS * (int64_t)shapeMax)
+        {
+            // Partners flagged, then counted in index order.
+            for (int32_t x = tid; x < shapeMax; x += NT)
+            {
+                s.planeFlag[x] = 0;
+            }
+            __syncthreads();
+            for (int32_t x = tid; x < c; x += NT)
+            {
+                s.planeFlag[(int32_t)(uint32_t)newKeys[a + x]] = 1;
+            }
+            __syncthreads();
+            BlockExclusiveScan<NT>(s.planeFlag, shapeMax);
+            for (int32_t x = tid; x < shapeMax; x += NT)
+            {
+                const int32_t at = s.planeFlag[x];
+                const int32_t next = x + 1 < shapeMax ? s.planeFlag[x + 1] : c;
+                if (next != at)
+                {
+                    newKeys[a + at] = (uint64_t)(uint32_t)row << 32 | (uint64_t)(uint32_t)x;
+                }
+            }
+            __syncthreads();
+            continue;
+        }
         for (int32_t x = tid; x < c; x += NT)
         {
             const uint64_t key = newKeys[a + x];
@@ -1167,12 +1407,44 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
     }
 }
 
-// A wide world's sweep (between m3BroadKernel PART 1 and PART 2): every
-// sorted position sweeps its own candidates, as the per-world kernel's
-// threads do, over the whole grid; row counts and the recorded pairs go
-// through global atomics (the fill orders each row afterwards).
-__global__ void __launch_bounds__(256) m3WideSweepKernel(const m3WorldView* views,
-                                                        const int32_t* order)
+// A wide world's broadphase before m3BroadKernel PART 2, over the whole
+// grid: head (counters), bounds with the move tests, a merge sort of the
+// sweep's elements (chunks in shared memory, then passes that double the
+// sorted runs), the gather of the sorted boxes with the move lists, and
+// the sweep.  One block for the first three took 0.75 ms a step at 10,000
+// bodies, and one thread a position left a heightfield's sweep over all
+// of them to one thread (3 ms).
+#define M3_WIDE_CHUNK 2048
+__global__ void m3WideHeadKernel(const m3WorldView* views, const int32_t* order, int32_t treeLag)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap, treeLag);
+    // The ring slot as in the per-world kernel: no moves are recorded
+    // unless this step reaches its containment tests.
+    int32_t slot = 0;
+    if (sc->treeTracked != 0)
+    {
+        slot = (int32_t)((uint32_t)sc->treeHead % (uint32_t)treeLag);
+        sc->treeHead += 1;
+        s.treeMoveCount[slot] = 0;
+    }
+    s.broadState[M3_BS_SLOT] = slot;
+    s.broadState[M3_BS_PLANES] = 0;
+    s.broadState[M3_BS_SWEEP] = 0;
+    s.broadState[M3_BS_PAIRS] = 0;
+    s.broadState[M3_BS_LONG] = 0;
+    // The wide kernels of this step start their grid barrier with no
+    // arrivals and no error.
+    s.gridBar[0] = 0;
+    s.gridBar[2] = 0;
+}
+
+// One shape a thread.  A block's moves are counted (planeFlag) and ranked
+// (treeMove: -1, or the rank among the block's moves).
+__global__ void __launch_bounds__(M3_BLOCK) m3WideBoundsKernel(const m3WorldView* views,
+                                                              const int32_t* order)
 {
     const m3WorldView& w = views[order[0]];
     m3WorldScalars* sc = w.sc;
@@ -1182,23 +1454,257 @@ __global__ void __launch_bounds__(256) m3WideSweepKernel(const m3WorldView* view
     }
     m3Scratch s;
     ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    const int32_t shapeMax = sc->shapeMax;
+    const int32_t i = blockIdx.x * M3_BLOCK + threadIdx.x;
+    const int32_t lane = threadIdx.x & 31;
+    const int32_t warp = threadIdx.x >> 5;
+    __shared__ int32_t warpMoves[M3_BLOCK / 32];
+    bool swept = false;
+    bool move = false;
+    uint64_t elem = M3_SWEEP_NONE;
+    if (i < shapeMax)
+    {
+        s.rowCount[i] = 0;
+        s.rowFill[i] = 0;
+        if (w.shapeAlive[i] != 0 && w.shapeType[i] == M3_SHAPE_PLANE)
+        {
+            const int32_t k = atomicAdd(&s.broadState[M3_BS_PLANES], 1);
+            if (k < M3_MAX_PLANES)
+            {
+                s.broadState[M3_BS_PLANE0 + k] = i;
+            }
+        }
+        else if (w.shapeAlive[i] != 0)
+        {
+            const m3Aabb b = ShapeBounds(w, i);
+            s.aabb[i] = b;
+            swept = true;
+            elem = SweepKey(b.lo[0], i);
+            if (sc->treeTracked != 0 && s.hasLeaf[i] != 0 && w.awake[w.shapeBody[i]] != 0)
+            {
+                const m3Aabb& leaf = s.leafBox[i];
+                move = !(leaf.lo[0] <= b.lo[0] && leaf.lo[1] <= b.lo[1] && leaf.lo[2] <= b.lo[2] &&
+                         b.hi[0] <= leaf.hi[0] && b.hi[1] <= leaf.hi[1] && b.hi[2] <= leaf.hi[2]);
+            }
+        }
+        s.sortKey[i] = elem;
+    }
+    const uint32_t moves = __ballot_sync(0xFFFFFFFFu, move);
+    const uint32_t sweeps = __ballot_sync(0xFFFFFFFFu, swept);
+    if (lane == 0)
+    {
+        warpMoves[warp] = __popc(moves);
+        if (sweeps != 0)
+        {
+            atomicAdd(&s.broadState[M3_BS_SWEEP], __popc(sweeps));
+        }
+    }
+    __syncthreads();
+    int32_t before = 0;
+    int32_t total = 0;
+    for (int32_t k = 0; k < M3_BLOCK / 32; ++k)
+    {
+        before += k < warp ? warpMoves[k] : 0;
+        total += warpMoves[k];
+    }
+    if (i < shapeMax)
+    {
+        s.treeMove[i] = move ? before + __popc(moves & ((1u << lane) - 1u)) : -1;
+    }
+    if (threadIdx.x == 0)
+    {
+        s.planeFlag[blockIdx.x] = total;
+    }
+}
+
+__global__ void __launch_bounds__(1024) m3WideChunkSortKernel(const m3WorldView* views,
+                                                             const int32_t* order)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    if (sc->status != 0)
+    {
+        return;
+    }
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    __shared__ uint64_t elems[M3_WIDE_CHUNK];
+    const int32_t base = blockIdx.x * M3_WIDE_CHUNK;
+    const int32_t n = sc->shapeMax - base;
+    for (int32_t i = threadIdx.x; i < M3_WIDE_CHUNK; i += 1024)
+    {
+        elems[i] = i < n ? s.sortKey[base + i] : M3_SWEEP_NONE;
+    }
+    __syncthreads();
+    BlockSort<1024>(elems, M3_WIDE_CHUNK);
+    for (int32_t i = threadIdx.x; i < M3_WIDE_CHUNK && i < n; i += 1024)
+    {
+        s.sortKey[base + i] = elems[i];
+    }
+}
+
+// One pass of the merge sort: runs of `run` sorted elements merge in pairs,
+// every element to its own place in its run plus its rank in the other
+// (equal elements, the padding, keep the first run's first).  `back` says
+// which of the two arrays holds the runs.
+__global__ void __launch_bounds__(M3_BLOCK) m3WideMergeKernel(const m3WorldView* views,
+                                                             const int32_t* order, int32_t run,
+                                                             int32_t back)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    if (sc->status != 0)
+    {
+        return;
+    }
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    uint64_t* spare = SweepSpare(s, sc->shapeCap);
+    const uint64_t* from = back != 0 ? spare : s.sortKey;
+    uint64_t* to = back != 0 ? s.sortKey : spare;
+    const int32_t n = sc->shapeMax;
+    const int32_t i = blockIdx.x * M3_BLOCK + threadIdx.x;
+    if (i >= n)
+    {
+        return;
+    }
+    const int32_t own = i / run * run;
+    const bool first = (i / run & 1) == 0;
+    const int32_t other = first ? own + run : own - run;
+    const uint64_t x = from[i];
+    int32_t lo = other < n ? other : n;
+    const int32_t start = lo;
+    int32_t hi = other + run < n ? other + run : n;
+    hi = hi > lo ? hi : lo;
+    while (lo < hi)
+    {
+        const int32_t mid = (lo + hi) >> 1;
+        const uint64_t y = from[mid];
+        if (first ? y < x : y <= x)
+        {
+            lo = mid + 1;
+        }
+        else
+        {
+            hi = mid;
+        }
+    }
+    to[(first ? own : other) + (i - own) + (lo - start)] = x;
+}
+
+// The sorted positions' boxes, and the step's move list in shape order
+// (each block's moves behind those of the blocks before it).
+__global__ void __launch_bounds__(M3_BLOCK) m3WideGatherKernel(const m3WorldView* views,
+                                                              const int32_t* order,
+                                                              int32_t treeLag, int32_t back)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    if (sc->status != 0)
+    {
+        return;
+    }
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap, treeLag);
     const int32_t n = s.broadState[M3_BS_SWEEP];
+    const int32_t planes = s.broadState[M3_BS_PLANES];
+    __shared__ int32_t s_before;
+    if (threadIdx.x == 0)
+    {
+        s_before = 0;
+    }
+    __syncthreads();
+    int32_t before = 0;
+    for (int32_t k = threadIdx.x; k < (int32_t)blockIdx.x; k += M3_BLOCK)
+    {
+        before += s.planeFlag[k];
+    }
+    atomicAdd(&s_before, before);
+    __syncthreads();
+    const int32_t i = blockIdx.x * M3_BLOCK + threadIdx.x;
+    const m3SweepBoxes boxes = SweepBoxes(s, sc->shapeCap);
+    if (i < n)
+    {
+        const uint64_t* from = back != 0 ? SweepSpare(s, sc->shapeCap) : s.sortKey;
+        PutSweepBox(s, boxes, i, (int32_t)(uint32_t)from[i]);
+    }
+    // Too many planes refuse the step before it moves any leaf.
+    const bool refused = planes > M3_MAX_PLANES;
+    if (!refused && i < sc->shapeMax && s.treeMove[i] >= 0)
+    {
+        const int64_t at = (int64_t)s.broadState[M3_BS_SLOT] * sc->shapeCap + s_before +
+                           s.treeMove[i];
+        m3Aabb fat = s.aabb[i];
+        for (int32_t k = 0; k < 3; ++k)
+        {
+            fat.lo[k] -= (double)M3_AABB_MARGIN;
+            fat.hi[k] += (double)M3_AABB_MARGIN;
+        }
+        s.treeMoveShape[at] = i;
+        s.treeMoveBox[at] = fat;
+        s.leafBox[i] = fat;
+    }
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1 && !refused)
+    {
+        s.treeMoveCount[s.broadState[M3_BS_SLOT]] = s_before + s.planeFlag[blockIdx.x];
+    }
+}
+
+__device__ __forceinline__ void WideRecord(const m3Scratch& s, int32_t pairCap, int32_t lo,
+                                           int32_t hi)
+{
+    atomicAdd(&s.rowCount[lo], 1);
+    const int32_t r = atomicAdd(&s.broadState[M3_BS_PAIRS], 1);
+    if (r < pairCap)
+    {
+        s.sweepPairs[r] = ((uint64_t)(uint32_t)lo << 32) | (uint64_t)(uint32_t)hi;
+    }
+}
+
+// The sweep, a warp a position; row counts and the recorded pairs go
+// through global atomics (the fill orders each row afterwards).  A
+// position with more candidates than M3_WIDE_LONG leaves the rest of them
+// to m3WideLongSweepKernel.
+#define M3_WIDE_LONG 1024
+__global__ void __launch_bounds__(M3_BLOCK) m3WideSweepKernel(const m3WorldView* views,
+                                                             const int32_t* order)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
     const int32_t planeCount = s.broadState[M3_BS_PLANES];
+    if (sc->status != 0 || planeCount > M3_MAX_PLANES)
+    {
+        return;
+    }
+    const int32_t n = s.broadState[M3_BS_SWEEP];
     const int32_t pairCap = sc->pairCap;
     const int32_t shapeMax = sc->shapeMax;
     const int32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t gstride = gridDim.x * blockDim.x;
-    int32_t* recorded = &s.broadState[M3_BS_PAIRS];
-    for (int32_t p = gtid; p < n; p += gstride)
+    const int32_t lane = threadIdx.x & 31;
+    const m3SweepBoxes boxes = SweepBoxes(s, sc->shapeCap);
+    for (int32_t p = gtid >> 5; p < n; p += gstride >> 5)
     {
-        SweepFrom(w, s, p, n, [&](int32_t lo, int32_t hi) {
-            atomicAdd(&s.rowCount[lo], 1);
-            const int32_t r = atomicAdd(recorded, 1);
-            if (r < pairCap)
-            {
-                s.sweepPairs[r] = ((uint64_t)(uint32_t)lo << 32) | (uint64_t)(uint32_t)hi;
-            }
-        });
+        const int32_t a = s.sortIdx[p];
+        const m3SweepBox boxA = GetSweepBox(boxes, p);
+        int32_t q = p + 1;
+        bool more = true;
+        while (more && q < n && q - p <= M3_WIDE_LONG)
+        {
+            const bool in = q + lane < n &&
+                            SweepPair(w, s, boxes, a, boxA, q + lane,
+                                      [&](int32_t lo, int32_t hi) { WideRecord(s, pairCap, lo, hi); });
+            more = __all_sync(0xFFFFFFFFu, in);
+            q += 32;
+        }
+        if (more && q < n && lane == 0)
+        {
+            const int32_t k = atomicAdd(&s.broadState[M3_BS_LONG], 1);
+            s.staticList[k] = p; // at most one entry a position
+            s.targetList[k] = q;
+        }
     }
     for (int32_t i = gtid; i < shapeMax; i += gstride)
     {
@@ -1217,6 +1723,66 @@ __global__ void __launch_bounds__(256) m3WideSweepKernel(const m3WorldView* view
             }
         }
     }
+}
+
+// The long sweeps' other candidates, M3_WIDE_LONG of them a block at a time.
+__global__ void __launch_bounds__(M3_BLOCK) m3WideLongSweepKernel(const m3WorldView* views,
+                                                                 const int32_t* order)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    if (sc->status != 0 || s.broadState[M3_BS_PLANES] > M3_MAX_PLANES)
+    {
+        return;
+    }
+    const int32_t n = s.broadState[M3_BS_SWEEP];
+    const int32_t pairCap = sc->pairCap;
+    const m3SweepBoxes boxes = SweepBoxes(s, sc->shapeCap);
+    const int64_t pieces = (n + M3_WIDE_LONG - 1) / M3_WIDE_LONG;
+    const int64_t units = pieces * s.broadState[M3_BS_LONG];
+    for (int64_t u = blockIdx.x; u < units; u += gridDim.x)
+    {
+        const int32_t k = (int32_t)(u / pieces);
+        const int32_t p = s.staticList[k];
+        const int32_t from = s.targetList[k] + (int32_t)(u % pieces) * M3_WIDE_LONG;
+        if (from >= n)
+        {
+            continue;
+        }
+        const int32_t a = s.sortIdx[p];
+        const m3SweepBox boxA = GetSweepBox(boxes, p);
+        const int32_t to = from + M3_WIDE_LONG < n ? from + M3_WIDE_LONG : n;
+        for (int32_t q = from + (int32_t)threadIdx.x; q < to; q += M3_BLOCK)
+        {
+            if (!SweepPair(w, s, boxes, a, boxA, q,
+                           [&](int32_t lo, int32_t hi) { WideRecord(s, pairCap, lo, hi); }))
+            {
+                break;
+            }
+        }
+    }
+}
+
+// The wide broadphase's launches before m3BroadKernel PART 2; how many.
+static int32_t LaunchWideSweep(const m3WorldView* views, const int32_t* order, int32_t shapeMax,
+                               int32_t smCount)
+{
+    const int32_t blocks = (shapeMax + M3_BLOCK - 1) / M3_BLOCK;
+    m3WideHeadKernel<<<1, 1>>>(views, order, M3_TREE_LAG);
+    m3WideBoundsKernel<<<blocks, M3_BLOCK>>>(views, order);
+    m3WideChunkSortKernel<<<(shapeMax + M3_WIDE_CHUNK - 1) / M3_WIDE_CHUNK, 1024>>>(views, order);
+    int32_t launches = 6;
+    int32_t back = 0;
+    for (int64_t run = M3_WIDE_CHUNK; run < shapeMax; run *= 2, back ^= 1, ++launches)
+    {
+        m3WideMergeKernel<<<blocks, M3_BLOCK>>>(views, order, (int32_t)run, back);
+    }
+    m3WideGatherKernel<<<blocks, M3_BLOCK>>>(views, order, M3_TREE_LAG, back);
+    m3WideSweepKernel<<<4 * smCount, M3_BLOCK>>>(views, order);
+    m3WideLongSweepKernel<<<4 * smCount, M3_BLOCK>>>(views, order);
+    return launches;
 }
 
 // Exclusive offsets of every world's new pair count, in batch order
@@ -4986,6 +5552,19 @@ static int32_t WideBlocks(const m3HostWorld* w)
     return blocks < maxResident ? blocks : maxResident;
 }
 
+// Elements the broadphase sorts in shared memory for worlds of at most
+// `shapes` shape slots: all of them up to 4096 (32 KB beside the kernel's
+// static arrays need no larger limit).
+static int32_t BroadSortCap(int32_t shapes)
+{
+    int32_t cap = 1;
+    while (cap < shapes && cap < 4096)
+    {
+        cap <<= 1;
+    }
+    return cap;
+}
+
 static void LaunchWideSubstep(const m3WorldView* views, const int32_t* order, float dt,
                               int32_t substeps, int32_t blocks)
 {
@@ -5547,6 +6126,13 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
         }
     }
     const cudaStream_t treeStream = s_classStreams.tree;
+    int32_t mostShapes = 1;
+    for (int32_t i = 0; i < count; ++i)
+    {
+        const int32_t shapes = worlds[i]->hv.sc->shapeMax;
+        mostShapes = shapes > mostShapes ? shapes : mostShapes;
+    }
+    const int32_t sortCap = BroadSortCap(mostShapes);
     // One large world alone: its substep loop over the whole grid.
     const int32_t wideBlocks = count == 1 ? WideBlocks(worlds[0]) : 0;
     for (int32_t step = 0; step < steps; ++step)
@@ -5589,19 +6175,17 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
         }
         if (wideBlocks > 0)
         {
-            // One large world: its sweep over the whole grid between the
-            // head and the tail of its broadphase.
-            m3BroadKernel<512, 1, 1><<<1, 512>>>(s_batch.dviews, s_batch.dorder, count,
-                                                  M3_TREE_LAG);
-            m3WideSweepKernel<<<4 * s_smCount, 256>>>(s_batch.dviews, s_batch.dorder);
+            // One large world: its bounds, sort and sweep over the whole
+            // grid, then the tail of its broadphase.
+            s_launches += LaunchWideSweep(s_batch.dviews, s_batch.dorder,
+                                          worlds[0]->hv.sc->shapeMax, s_smCount);
             m3BroadKernel<512, 1, 2><<<1, 512>>>(s_batch.dviews, s_batch.dorder, count,
-                                                  M3_TREE_LAG);
-            s_launches += 2;
+                                                  M3_TREE_LAG, 0);
         }
         else
         {
-            m3BroadKernel<M3_BLOCK, 2><<<count, M3_BLOCK>>>(s_batch.dviews, s_batch.dorder, count,
-                                                            M3_TREE_LAG);
+            m3BroadKernel<M3_BLOCK, 2><<<count, M3_BLOCK, sortCap * sizeof(uint64_t)>>>(
+                s_batch.dviews, s_batch.dorder, count, M3_TREE_LAG, sortCap);
         }
         cudaEventRecord(ev[1]);
         if (anyTracked)
@@ -5909,7 +6493,9 @@ extern "C" int32_t m3gpu_step_world_noalloc(m3WorldId worldId, float dt, int32_t
     m3gpuWaitTree(w);
     w->leafBoxValid = false;
     m3LeafBoxKernel<<<1, M3_BLOCK>>>(sym.view, 1);
-    m3BroadKernel<M3_BLOCK, 1><<<1, M3_BLOCK>>>(sym.view, order, 1, 1);
+    const int32_t sortCap = BroadSortCap(w->hv.sc->shapeMax);
+    m3BroadKernel<M3_BLOCK, 1><<<1, M3_BLOCK, sortCap * sizeof(uint64_t)>>>(sym.view, order, 1, 1,
+                                                                            sortCap);
     m3TreeKernel<<<1, M3_TREE_THREADS>>>(sym.view, order, 1, 1, sym.table + 3);
     m3PairOffsetsKernel<<<1, M3_BLOCK>>>(sym.view, 1, offsets);
     m3NarrowKernel<<<148, 128>>>(sym.view, offsets, 1);
