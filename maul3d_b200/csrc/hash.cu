@@ -32,6 +32,15 @@
 // bytes) and hashes the staged bytes tile by tile, carrying (lo, hi)
 // across tiles and rounds.  The
 // result is bit-identical to m3WorldHashView.
+//
+// A large world among few is hashed over many blocks instead (one block
+// took 36 ms for a world of 20,000 bodies, 46,000 joints and 121,000 pairs,
+// on one SM of 148): its stream is written out once, and each of the
+// facts above becomes a pass over the stream's 8 KB tiles, a block a
+// tile: eight passes for the low byte's bits (a tile's bit toggles are
+// one parity, and a tile's start is the parity of the tiles before it),
+// one for the tiles' lo maps, one for their hi maps, and one block that
+// composes them.
 #include "m3_world.h"
 #include "m3_hash.h"
 
@@ -39,7 +48,11 @@
 
 #define M3H_BLOCK 256
 #define M3H_WARPS (M3H_BLOCK / 32)
-#define M3H_RECORD_MAX 256 // longest record of the stream (a body: 197 bytes)
+#define M3H_RECORD_MAX 256 // longest record of the stream
+// The longest record of each kind (m3_hash.h, every optional field there).
+#define M3H_BODY_MAX 196
+#define M3H_SHAPE_MAX 125
+#define M3H_JOINT_MAX 171
 // Records staged per round: half the block, so that the stage (32 KB)
 // lets four blocks share an SM (the registers allow four; a 64 KB stage
 // allowed three).
@@ -193,76 +206,87 @@ __device__ void AffineBlockScan(uint32_t A, uint32_t C, uint32_t* exA, uint32_t*
     *totC = tC;
 }
 
-// Folds tile[0, n) (n <= M3H_TILE) into (lo, hi); every thread of the
-// block calls it with the same arguments and gets the same result.
-__device__ void FnvTile(const uint8_t* tile, int32_t n, uint32_t& lo, uint32_t& hi,
-                        m3HashShared& sh)
+// One thread's 32-byte chunk of a tile of n bytes: its words, its bit
+// planes (bit i of B[j] = bit j of byte i) and which bytes exist.
+struct m3HashChunk
+{
+    uint32_t wd[8];
+    uint32_t B[8];
+    uint32_t valid;
+    int32_t cnt;
+};
+
+__device__ __forceinline__ void LoadChunk(const uint8_t* tile, int32_t n, m3HashChunk& c)
 {
     const int32_t tid = threadIdx.x;
-    const int32_t lane = tid & 31;
-    const int32_t warp = tid >> 5;
     int32_t cnt = n - tid * M3H_CHUNK;
     cnt = cnt < 0 ? 0 : (cnt > M3H_CHUNK ? M3H_CHUNK : cnt);
-    const uint32_t valid = cnt >= 32 ? 0xFFFFFFFFu : ((1u << cnt) - 1u);
-
-    uint32_t wd[8];
+    c.cnt = cnt;
+    c.valid = cnt >= 32 ? 0xFFFFFFFFu : ((1u << cnt) - 1u);
     if (cnt > 0)
     {
         const uint4* src = (const uint4*)(tile + tid * M3H_CHUNK);
         const uint4 q0 = src[0];
         const uint4 q1 = src[1];
-        wd[0] = q0.x;
-        wd[1] = q0.y;
-        wd[2] = q0.z;
-        wd[3] = q0.w;
-        wd[4] = q1.x;
-        wd[5] = q1.y;
-        wd[6] = q1.z;
-        wd[7] = q1.w;
+        c.wd[0] = q0.x;
+        c.wd[1] = q0.y;
+        c.wd[2] = q0.z;
+        c.wd[3] = q0.w;
+        c.wd[4] = q1.x;
+        c.wd[5] = q1.y;
+        c.wd[6] = q1.z;
+        c.wd[7] = q1.w;
     }
     else
     {
 #pragma unroll
         for (int32_t k = 0; k < 8; ++k)
         {
-            wd[k] = 0u;
+            c.wd[k] = 0u;
         }
     }
-    // Bit planes: bit i of B[j] = bit j of byte i of the chunk.
-    uint32_t B[8];
 #pragma unroll
     for (int32_t j = 0; j < 8; ++j)
     {
-        B[j] = 0u;
+        c.B[j] = 0u;
     }
 #pragma unroll
     for (int32_t g = 0; g < 4; ++g)
     {
-        const uint64_t y = Transpose8((uint64_t)wd[2 * g] | ((uint64_t)wd[2 * g + 1] << 32));
+        const uint64_t y = Transpose8((uint64_t)c.wd[2 * g] | ((uint64_t)c.wd[2 * g + 1] << 32));
 #pragma unroll
         for (int32_t j = 0; j < 8; ++j)
         {
-            B[j] |= (uint32_t)((y >> (8 * j)) & 0xFFu) << (8 * g);
+            c.B[j] |= (uint32_t)((y >> (8 * j)) & 0xFFu) << (8 * g);
         }
     }
+}
 
-    // Round j: bit j of the low byte s before every byte of the tile.
+// Rounds 0 .. ROUNDS - 1: plane j of S is bit j of the low byte before
+// every byte of the tile, which starts at the low byte s0 (its bits below
+// ROUNDS matter).  Returns the parity of the tile's toggles in the last
+// round's bit.
+template <int ROUNDS>
+__device__ __forceinline__ uint32_t LowPlanes(const m3HashChunk& chunk, uint32_t s0, uint32_t S[8],
+                                              m3HashShared& sh)
+{
+    const int32_t lane = threadIdx.x & 31;
+    const int32_t warp = threadIdx.x >> 5;
     // acc holds, bit-sliced, ((s ^ b) mod 2^j) * 435 mod 256 for every
     // byte, i.e. the part of the product known from the lower bits.
     uint32_t acc[8];
-    uint32_t S[8];
 #pragma unroll
     for (int32_t j = 0; j < 8; ++j)
     {
         acc[j] = 0u;
     }
-    const uint32_t s0 = lo & 0xFFu;
+    uint32_t parity = 0u;
     const uint32_t ltMask = (1u << lane) - 1u;
 #pragma unroll
-    for (int32_t j = 0; j < 8; ++j)
+    for (int32_t j = 0; j < ROUNDS; ++j)
     {
         // s'_j = s_j ^ b_j ^ acc_j: the toggles, prefix-XORed.
-        const uint32_t T = (B[j] ^ acc[j]) & valid;
+        const uint32_t T = (chunk.B[j] ^ acc[j]) & chunk.valid;
         uint32_t Q = T << 1;
         Q ^= Q << 1;
         Q ^= Q << 2;
@@ -275,6 +299,13 @@ __device__ void FnvTile(const uint8_t* tile, int32_t n, uint32_t& lo, uint32_t& 
             sh.warpBits[j][warp] = (uint32_t)(__popc(ballot) & 1);
         }
         __syncthreads();
+        if (j == ROUNDS - 1)
+        {
+            for (int32_t k = 0; k < M3H_WARPS; ++k)
+            {
+                parity ^= sh.warpBits[j][k];
+            }
+        }
         uint32_t carry = ((s0 >> j) & 1u) ^ ((uint32_t)__popc(ballot & ltMask) & 1u);
         for (int32_t k = 0; k < warp; ++k)
         {
@@ -283,7 +314,7 @@ __device__ void FnvTile(const uint8_t* tile, int32_t n, uint32_t& lo, uint32_t& 
         S[j] = Q ^ (0u - carry);
         // Add x_j * 435 * 2^j (435 = 0b110110011 = 256 + 179; mod 256 the
         // multiplier is 179 = 2^7 + 2^5 + 2^4 + 2^1 + 2^0).
-        const uint32_t X = S[j] ^ B[j];
+        const uint32_t X = S[j] ^ chunk.B[j];
 #pragma unroll
         for (int32_t o = 0; o < 8; ++o)
         {
@@ -301,6 +332,13 @@ __device__ void FnvTile(const uint8_t* tile, int32_t n, uint32_t& lo, uint32_t& 
             }
         }
     }
+    return parity;
+}
+
+// The chunk's lo map from its low-byte planes: lo' = 435 * (lo + ((s ^ b)
+// - s)) per byte, A lo + C in all (A is 435 to the chunk's length).
+__device__ __forceinline__ uint32_t ChunkLo(const m3HashChunk& chunk, const uint32_t S[8])
+{
     // Low bytes back to byte order.
     uint32_t sw[8];
 #pragma unroll
@@ -316,44 +354,77 @@ __device__ void FnvTile(const uint8_t* tile, int32_t n, uint32_t& lo, uint32_t& 
         sw[2 * g] = (uint32_t)y;
         sw[2 * g + 1] = (uint32_t)(y >> 32);
     }
-    // lo: lo' = 435 * (lo + ((s ^ b) - s)), one affine map per chunk.
     uint32_t C = 0u;
 #pragma unroll
     for (int32_t k = 0; k < M3H_CHUNK; ++k)
     {
-        if (k < cnt)
+        if (k < chunk.cnt)
         {
             const uint32_t s = (sw[k >> 2] >> (8 * (k & 3))) & 0xFFu;
-            const uint32_t b = (wd[k >> 2] >> (8 * (k & 3))) & 0xFFu;
+            const uint32_t b = (chunk.wd[k >> 2] >> (8 * (k & 3))) & 0xFFu;
             C = M3H_MUL * (C + ((s ^ b) - s));
         }
     }
-    const uint32_t A = sh.pow435[cnt];
+    return C;
+}
+
+// The chunk's hi map from lo before it: hi' = 435 * hi + umulhi(x, 435) +
+// (x << 8) per byte with x = lo ^ b.
+__device__ __forceinline__ uint32_t ChunkHi(const m3HashChunk& chunk, uint32_t lo)
+{
+    uint32_t H = 0u;
+#pragma unroll
+    for (int32_t k = 0; k < M3H_CHUNK; ++k)
+    {
+        if (k < chunk.cnt)
+        {
+            const uint32_t b = (chunk.wd[k >> 2] >> (8 * (k & 3))) & 0xFFu;
+            const uint32_t x = lo ^ b;
+            H = M3H_MUL * H + (__umulhi(x, M3H_MUL) + (x << 8));
+            lo = x * M3H_MUL;
+        }
+    }
+    return H;
+}
+
+// Folds tile[0, n) (n <= M3H_TILE) into (lo, hi); every thread of the
+// block calls it with the same arguments and gets the same result.
+__device__ void FnvTile(const uint8_t* tile, int32_t n, uint32_t& lo, uint32_t& hi,
+                        m3HashShared& sh)
+{
+    m3HashChunk chunk;
+    uint32_t S[8];
+    LoadChunk(tile, n, chunk);
+    LowPlanes<8>(chunk, lo & 0xFFu, S, sh);
+    const uint32_t C = ChunkLo(chunk, S);
+    const uint32_t A = sh.pow435[chunk.cnt];
     uint32_t exA;
     uint32_t exC;
     uint32_t totA;
     uint32_t totC;
     AffineBlockScan(A, C, &exA, &exC, &totA, &totC, sh);
-    uint32_t l = exA * lo + exC;
+    const uint32_t H = ChunkHi(chunk, exA * lo + exC);
     const uint32_t loEnd = totA * lo + totC;
-    // hi: hi' = 435 * hi + umulhi(x, 435) + (x << 8), x = lo ^ b.
-    uint32_t H = 0u;
-#pragma unroll
-    for (int32_t k = 0; k < M3H_CHUNK; ++k)
-    {
-        if (k < cnt)
-        {
-            const uint32_t b = (wd[k >> 2] >> (8 * (k & 3))) & 0xFFu;
-            const uint32_t x = l ^ b;
-            H = M3H_MUL * H + (__umulhi(x, M3H_MUL) + (x << 8));
-            l = x * M3H_MUL;
-        }
-    }
     uint32_t hA;
     uint32_t hC;
     AffineBlockScan(A, H, &exA, &exC, &hA, &hC, sh);
     lo = loEnd;
     hi = hA * hi + hC;
+}
+
+// The powers of 435 a chunk's length needs; read after a barrier.
+__device__ __forceinline__ void HashPowers(m3HashShared& sh)
+{
+    const int32_t tid = threadIdx.x;
+    if (tid <= M3H_CHUNK)
+    {
+        uint32_t p = 1u;
+        for (int32_t k = 0; k < tid; ++k)
+        {
+            p *= M3H_MUL;
+        }
+        sh.pow435[tid] = p;
+    }
 }
 
 __global__ void __launch_bounds__(M3H_BLOCK, 5) m3HashKernel(const m3WorldView* views,
@@ -365,15 +436,7 @@ __global__ void __launch_bounds__(M3H_BLOCK, 5) m3HashKernel(const m3WorldView* 
     extern __shared__ __align__(16) uint8_t s_stage[];
     __shared__ m3HashShared sh;
     const int32_t tid = threadIdx.x;
-    if (tid <= M3H_CHUNK)
-    {
-        uint32_t p = 1u;
-        for (int32_t k = 0; k < tid; ++k)
-        {
-            p *= M3H_MUL;
-        }
-        sh.pow435[tid] = p;
-    }
+    HashPowers(sh);
     if (tid == 0)
     {
         sh.bad = 0;
@@ -417,6 +480,382 @@ __global__ void __launch_bounds__(M3H_BLOCK, 5) m3HashKernel(const m3WorldView* 
     {
         out[wi] = sh.bad != 0 ? 0ull : (((uint64_t)hi << 32) | lo);
     }
+}
+
+// ---------------------------------------------------------------------
+// Large worlds over many blocks.  blockIdx.y is the world's job, the
+// blocks of a row stride over its record blocks or tiles.  The job's
+// working words: [0] the stream's bytes, then one sum per record block,
+// eight bit arrays of the tiles' parities, and the tiles' maps.
+// ---------------------------------------------------------------------
+struct m3HashWork
+{
+    uint32_t* bytes;
+    uint32_t* sums;  // per M3H_ROUND_RECORDS records: their bytes
+    uint32_t* bits;  // 8 arrays of `words`: a tile's parity a bit
+    uint32_t* mapA;  // per tile: lo' = A lo + C, hi' = A hi + H
+    uint32_t* mapC;
+    uint32_t* mapH;
+    int32_t words;
+};
+
+// The stream's bytes; a stream beyond the job's tiles cannot happen with
+// this record set (it would end as the hash 0, and never overrun them).
+__device__ __forceinline__ int32_t StreamBytes(const m3HashJob& job, const m3HashWork& work)
+{
+    const uint32_t cap = (uint32_t)job.tiles * M3H_TILE;
+    return (int32_t)(*work.bytes < cap ? *work.bytes : cap);
+}
+
+__device__ __forceinline__ m3HashWork HashWork(const m3HashJob& job)
+{
+    const int32_t tiles = job.tiles;
+    m3HashWork k;
+    k.words = (tiles + 31) / 32;
+    k.bytes = job.work;
+    k.sums = job.work + 8;
+    k.bits = k.sums + job.recordBlocks;
+    k.mapA = k.bits + 8 * k.words;
+    k.mapC = k.mapA + tiles;
+    k.mapH = k.mapC + tiles;
+    return k;
+}
+
+// Words of a job of at most `tiles` tiles and `recordBlocks` record blocks.
+static int64_t HashWorkWords(int64_t tiles, int64_t recordBlocks)
+{
+    return 8 + recordBlocks + 8 * ((tiles + 31) / 32) + 3 * tiles;
+}
+
+__global__ void __launch_bounds__(M3H_BLOCK) m3HashLengthKernel(const __grid_constant__ m3HashJobs jobs)
+{
+    const m3HashJob& job = jobs.job[blockIdx.y];
+    const m3WorldView* w = job.view;
+    const m3HashWork work = HashWork(job);
+    __shared__ int32_t s_warp[M3H_WARPS];
+    const int32_t records = m3HashRecordCount(w);
+    const int32_t lane = threadIdx.x & 31;
+    const int32_t warp = threadIdx.x >> 5;
+    for (int32_t i = blockIdx.x * M3H_BLOCK + threadIdx.x; i < 8 * work.words;
+         i += gridDim.x * M3H_BLOCK)
+    {
+        work.bits[i] = 0u;
+    }
+    for (int32_t r0 = blockIdx.x * M3H_BLOCK; r0 < records; r0 += gridDim.x * M3H_BLOCK)
+    {
+        const int32_t r = r0 + threadIdx.x;
+        int32_t len = 0;
+        if (r < records)
+        {
+            m3CountSink c{0};
+            m3HashRecord(w, r, c);
+            len = c.n;
+        }
+        for (int32_t o = 16; o > 0; o >>= 1)
+        {
+            len += __shfl_xor_sync(0xFFFFFFFFu, len, o);
+        }
+        if (lane == 0)
+        {
+            s_warp[warp] = len;
+        }
+        __syncthreads();
+        const int32_t half = M3H_WARPS / 2;
+        if (threadIdx.x < 2 && r0 + (int32_t)threadIdx.x * M3H_ROUND_RECORDS < records)
+        {
+            int32_t sum = 0;
+            for (int32_t k = 0; k < half; ++k)
+            {
+                sum += s_warp[threadIdx.x * half + k];
+            }
+            work.sums[r0 / M3H_ROUND_RECORDS + threadIdx.x] = (uint32_t)sum;
+        }
+        __syncthreads();
+    }
+}
+
+// Sum of v over the block, the same in every thread.
+__device__ uint32_t HashBlockSum(uint32_t v, m3HashShared& sh)
+{
+    for (int32_t o = 16; o > 0; o >>= 1)
+    {
+        v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+        sh.warpA[threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    uint32_t all = 0;
+    for (int32_t k = 0; k < M3H_WARPS; ++k)
+    {
+        all += sh.warpA[k];
+    }
+    __syncthreads();
+    return all;
+}
+
+// Writes the stream: a record block is laid out in shared memory at its
+// place's alignment, then copied 16 bytes at a time.
+__global__ void __launch_bounds__(M3H_BLOCK) m3HashStreamKernel(const __grid_constant__ m3HashJobs jobs)
+{
+    const m3HashJob& job = jobs.job[blockIdx.y];
+    const m3WorldView* w = job.view;
+    const m3HashWork work = HashWork(job);
+    extern __shared__ __align__(16) uint8_t s_stage[];
+    __shared__ m3HashShared sh;
+    const int32_t tid = threadIdx.x;
+    const int32_t records = m3HashRecordCount(w);
+    const int32_t recordBlocks = (records + M3H_ROUND_RECORDS - 1) / M3H_ROUND_RECORDS;
+    for (int32_t rb = blockIdx.x; rb < recordBlocks; rb += gridDim.x)
+    {
+        uint32_t before = 0;
+        for (int32_t k = tid; k < rb; k += M3H_BLOCK)
+        {
+            before += work.sums[k];
+        }
+        const uint32_t base = HashBlockSum(before, sh);
+        const int32_t r = rb * M3H_ROUND_RECORDS + tid;
+        int32_t len = 0;
+        if (tid < M3H_ROUND_RECORDS && r < records)
+        {
+            m3CountSink c{0};
+            m3HashRecord(w, r, c);
+            len = c.n;
+        }
+        int32_t total = 0;
+        const int32_t off = HashBlockScan(len, &total, sh);
+        const int32_t shift = (int32_t)(base & 15u);
+        if (len > 0)
+        {
+            m3StageSink k{s_stage + shift, off};
+            m3HashRecord(w, r, k);
+        }
+        __syncthreads();
+        // Stream bytes [base, base + total) = stage bytes [shift, end).
+        uint8_t* to = job.stream + (base - (uint32_t)shift);
+        const bool fits = (int64_t)base + total <= (int64_t)job.tiles * M3H_TILE;
+        const int32_t end = fits ? shift + total : shift;
+        const int32_t head = shift == 0 ? 0 : 16;
+        const int32_t tail = end & ~15;
+        for (int32_t k = head + 16 * tid; k < tail; k += 16 * M3H_BLOCK)
+        {
+            *(uint4*)(to + k) = *(const uint4*)(s_stage + k);
+        }
+        if (tid < 16 && tid >= shift && tid < head && tid < end)
+        {
+            to[tid] = s_stage[tid];
+        }
+        if (tid >= 16 && tid < 32 && tail >= head && tail + tid - 16 < end)
+        {
+            to[tail + tid - 16] = s_stage[tail + tid - 16];
+        }
+        if (rb == recordBlocks - 1 && tid == 0)
+        {
+            *work.bytes = base + (uint32_t)total;
+        }
+        __syncthreads();
+    }
+}
+
+// The low byte's bits below BITS at the start of tile t: the parities of
+// the tiles before it, on the stream's first low byte (warp j counts bit j).
+template <int BITS>
+__device__ uint32_t TileLow(const m3HashWork& work, int32_t t, m3HashShared& sh)
+{
+    const int32_t lane = threadIdx.x & 31;
+    const int32_t warp = threadIdx.x >> 5;
+    uint32_t odd = 0;
+    if (warp < BITS)
+    {
+        const uint32_t* bits = work.bits + warp * work.words;
+        for (int32_t k = lane; k <= t >> 5; k += 32)
+        {
+            const uint32_t mask = k < t >> 5 ? 0xFFFFFFFFu : (1u << (t & 31)) - 1u;
+            odd ^= (uint32_t)__popc(bits[k] & mask) & 1u;
+        }
+        odd = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, odd != 0)) & 1u;
+    }
+    if (lane == 0)
+    {
+        sh.warpC[warp] = odd << warp;
+    }
+    __syncthreads();
+    uint32_t low = (uint32_t)M3_HASH_INIT & 0xFFu;
+    for (int32_t k = 0; k < M3H_WARPS; ++k)
+    {
+        low ^= sh.warpC[k];
+    }
+    __syncthreads();
+    return low;
+}
+
+template <int BIT>
+__global__ void __launch_bounds__(M3H_BLOCK) m3HashBitKernel(const __grid_constant__ m3HashJobs jobs)
+{
+    const m3HashJob& job = jobs.job[blockIdx.y];
+    const m3HashWork work = HashWork(job);
+    __shared__ m3HashShared sh;
+    const int32_t bytes = StreamBytes(job, work);
+    for (int32_t t = blockIdx.x; t * (int64_t)M3H_TILE < bytes; t += gridDim.x)
+    {
+        const int32_t base = t * M3H_TILE;
+        const uint32_t low = TileLow<BIT>(work, t, sh);
+        m3HashChunk chunk;
+        uint32_t S[8];
+        LoadChunk(job.stream + base, bytes - base < M3H_TILE ? bytes - base : M3H_TILE, chunk);
+        const uint32_t parity = LowPlanes<BIT + 1>(chunk, low, S, sh);
+        if (threadIdx.x == 0 && parity != 0)
+        {
+            atomicOr(&work.bits[BIT * work.words + (t >> 5)], 1u << (t & 31));
+        }
+        __syncthreads();
+    }
+}
+
+// Each tile's lo map (HI false), or its hi map from the lo its start has
+// (the maps of the tiles before it, composed).
+template <bool HI>
+__global__ void __launch_bounds__(M3H_BLOCK) m3HashMapKernel(const __grid_constant__ m3HashJobs jobs)
+{
+    const m3HashJob& job = jobs.job[blockIdx.y];
+    const m3HashWork work = HashWork(job);
+    __shared__ m3HashShared sh;
+    HashPowers(sh);
+    __syncthreads();
+    const int32_t bytes = StreamBytes(job, work);
+    for (int32_t t = blockIdx.x; t * (int64_t)M3H_TILE < bytes; t += gridDim.x)
+    {
+        const int32_t base = t * M3H_TILE;
+        uint32_t exA;
+        uint32_t exC;
+        uint32_t totA;
+        uint32_t totC;
+        uint32_t lo = (uint32_t)M3_HASH_INIT;
+        if (HI)
+        {
+            const int32_t per = (t + M3H_BLOCK - 1) / M3H_BLOCK;
+            uint32_t A = 1u;
+            uint32_t C = 0u;
+            for (int32_t k = threadIdx.x * per; k < ((int32_t)threadIdx.x + 1) * per && k < t; ++k)
+            {
+                C = work.mapA[k] * C + work.mapC[k];
+                A = work.mapA[k] * A;
+            }
+            AffineBlockScan(A, C, &exA, &exC, &totA, &totC, sh);
+            lo = totA * lo + totC;
+        }
+        const uint32_t low = TileLow<8>(work, t, sh);
+        m3HashChunk chunk;
+        uint32_t S[8];
+        LoadChunk(job.stream + base, bytes - base < M3H_TILE ? bytes - base : M3H_TILE, chunk);
+        LowPlanes<8>(chunk, low, S, sh);
+        const uint32_t A = sh.pow435[chunk.cnt];
+        AffineBlockScan(A, ChunkLo(chunk, S), &exA, &exC, &totA, &totC, sh);
+        if (HI)
+        {
+            AffineBlockScan(A, ChunkHi(chunk, exA * lo + exC), &exA, &exC, &totA, &totC, sh);
+        }
+        if (threadIdx.x == 0)
+        {
+            work.mapA[t] = totA;
+            (HI ? work.mapH : work.mapC)[t] = totC;
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(M3H_BLOCK) m3HashFinalKernel(const __grid_constant__ m3HashJobs jobs)
+{
+    const m3HashJob& job = jobs.job[blockIdx.x];
+    const m3HashWork work = HashWork(job);
+    __shared__ m3HashShared sh;
+    const int32_t tiles = (StreamBytes(job, work) + M3H_TILE - 1) / M3H_TILE;
+    const int32_t per = (tiles + M3H_BLOCK - 1) / M3H_BLOCK;
+    uint32_t A = 1u;
+    uint32_t C = 0u;
+    uint32_t H = 0u;
+    for (int32_t k = threadIdx.x * per; k < ((int32_t)threadIdx.x + 1) * per && k < tiles; ++k)
+    {
+        C = work.mapA[k] * C + work.mapC[k];
+        H = work.mapA[k] * H + work.mapH[k];
+        A = work.mapA[k] * A;
+    }
+    uint32_t exA;
+    uint32_t exC;
+    uint32_t totA;
+    uint32_t loC;
+    uint32_t hiC;
+    AffineBlockScan(A, C, &exA, &exC, &totA, &loC, sh);
+    AffineBlockScan(A, H, &exA, &exC, &totA, &hiC, sh);
+    if (threadIdx.x == 0)
+    {
+        const uint32_t lo = totA * (uint32_t)M3_HASH_INIT + loC;
+        const uint32_t hi = totA * (uint32_t)(M3_HASH_INIT >> 32) + hiC;
+        *job.out = *work.bytes <= (uint32_t)job.tiles * M3H_TILE ? ((uint64_t)hi << 32) | lo : 0ull;
+    }
+}
+
+// Fills in a job's sizes; false when the working memory cannot hold the
+// world's longest stream.
+bool m3gpuHashJobFits(m3HashJob* job, int64_t streamBytes, int64_t workBytes, int64_t bodies,
+                      int64_t shapes, int64_t joints, int64_t pairs)
+{
+    const int64_t records = 2 + bodies + shapes + joints + pairs;
+    const int64_t bytes = 2 * M3H_RECORD_MAX + M3H_BODY_MAX * bodies + M3H_SHAPE_MAX * shapes +
+                          M3H_JOINT_MAX * joints +
+                          (int64_t)(sizeof(uint64_t) + sizeof(m3Manifold)) * pairs;
+    const int64_t tiles = (bytes + M3H_TILE - 1) / M3H_TILE;
+    const int64_t recordBlocks = (records + M3H_ROUND_RECORDS - 1) / M3H_ROUND_RECORDS;
+    job->tiles = (int32_t)tiles;
+    job->recordBlocks = (int32_t)recordBlocks;
+    // The last tile's chunks are read whole.
+    return bytes < INT32_MAX - M3H_TILE && tiles * M3H_TILE <= streamBytes &&
+           4 * HashWorkWords(tiles, recordBlocks) <= workBytes;
+}
+
+// Launches the passes of `count` jobs; the number of kernels, or a negative
+// error code.
+int32_t m3gpuLaunchHashJobs(const m3HashJobs& jobs, int32_t count)
+{
+    static int s_configured = -1;
+    const int32_t stage = M3H_STAGE_BYTES + 16;
+    int device = 0;
+    cudaGetDevice(&device);
+    if (s_configured != device)
+    {
+        const cudaError_t e = cudaFuncSetAttribute(
+            m3HashStreamKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, stage);
+        if (e != cudaSuccess)
+        {
+            return -m3gpuSetError(M3GPU_ERR_CUDA, "cudaFuncSetAttribute(hash stage): %s",
+                                  cudaGetErrorString(e));
+        }
+        s_configured = device;
+    }
+    // Blocks a job: all of its tiles at once, up to four blocks an SM over
+    // the jobs.
+    int32_t most = 1;
+    for (int32_t k = 0; k < count; ++k)
+    {
+        most = jobs.job[k].tiles > most ? jobs.job[k].tiles : most;
+    }
+    const int32_t share = (148 * 4 + count - 1) / count;
+    const dim3 grid((uint32_t)(most < share ? most : share), (uint32_t)count);
+    m3HashLengthKernel<<<grid, M3H_BLOCK>>>(jobs);
+    m3HashStreamKernel<<<grid, M3H_BLOCK, stage>>>(jobs);
+    m3HashBitKernel<0><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<1><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<2><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<3><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<4><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<5><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<6><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashBitKernel<7><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashMapKernel<false><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashMapKernel<true><<<grid, M3H_BLOCK>>>(jobs);
+    m3HashFinalKernel<<<count, M3H_BLOCK>>>(jobs);
+    return 13;
 }
 
 int32_t m3gpuLaunchHash(const m3WorldView* views, const int32_t* order, int32_t count,

@@ -430,6 +430,26 @@ void m3gpuWaitTree(m3HostWorld* w);
 // `order`, out[world] = that world's m3WorldHashView.
 int32_t m3gpuLaunchHash(const m3WorldView* views, const int32_t* order, int32_t count,
                         uint64_t* out);
+// A large world hashed over many blocks: its view and hash on the device,
+// and the device memory for its byte stream and the passes' words (sizes
+// by m3gpuHashJobFits).
+#define M3_HASH_JOBS 64
+struct m3HashJob
+{
+    const m3WorldView* view;
+    uint8_t* stream;
+    uint32_t* work;
+    uint64_t* out;
+    int32_t tiles;
+    int32_t recordBlocks;
+};
+struct m3HashJobs
+{
+    m3HashJob job[M3_HASH_JOBS];
+};
+bool m3gpuHashJobFits(m3HashJob* job, int64_t streamBytes, int64_t workBytes, int64_t bodies,
+                      int64_t shapes, int64_t joints, int64_t pairs);
+int32_t m3gpuLaunchHashJobs(const m3HashJobs& jobs, int32_t count);
 
 // Error reporting (capi.cpp).
 int32_t m3gpuSetError(int32_t code, const char* fmt, ...);

@@ -6307,6 +6307,26 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
     return M3GPU_OK;
 }
 
+// A world large enough to be hashed over many blocks: thirteen launches
+// take about 60 us, one block about 0.17 us a record, and a world has about
+// as many pairs as bodies and shapes together.
+#define M3_HASH_WIDE_RECORDS 256
+static bool HashJobOf(const m3HostWorld* w, m3HashJob* job)
+{
+    const m3WorldScalars* sc = w->hv.sc;
+    if (sc->bodyMax + sc->shapeMax + sc->jointMax < M3_HASH_WIDE_RECORDS)
+    {
+        return false;
+    }
+    m3Scratch s;
+    ScratchCarve(&s, w->dv.scratch, w->bodyCap, w->shapeCap, w->jointCap, w->pairCap);
+    job->stream = (uint8_t*)s.rows.ro;
+    job->work = (uint32_t*)s.rows.acc;
+    return m3gpuHashJobFits(job, (int64_t)sizeof(float) * M3C_WORDS * s.rows.stride,
+                            (int64_t)sizeof(float) * M3A_WORDS * s.rows.stride, sc->bodyMax,
+                            sc->shapeMax, sc->jointMax, w->pairCap);
+}
+
 int32_t m3gpuHashBatch(m3HostWorld** worlds, int32_t count, uint64_t* out)
 {
     M3_DEVICE_GUARD;
@@ -6320,12 +6340,44 @@ int32_t m3gpuHashBatch(m3HostWorld** worlds, int32_t count, uint64_t* out)
     {
         return rc;
     }
-    rc = m3gpuLaunchHash(s_batch.dviews, s_batch.dorder, count, s_batch.dhash);
+    // The large worlds over many blocks each (their stream and words in the
+    // contact rows' memory, which a step fills before it reads it), the
+    // others a block each.  With more large worlds than M3_HASH_JOBS a block
+    // each fills the GPU as well.
+    m3HashJobs jobs;
+    int32_t large = 0;
+    for (; large < count; ++large)
+    {
+        const int32_t wi = s_batch.horder[(size_t)large];
+        m3HashJob job;
+        if (!HashJobOf(worlds[wi], &job))
+        {
+            break;
+        }
+        if (large == M3_HASH_JOBS)
+        {
+            large = 0;
+            break;
+        }
+        job.view = s_batch.dviews + wi;
+        job.out = s_batch.dhash + wi;
+        jobs.job[large] = job;
+    }
+    if (large > 0)
+    {
+        const int32_t launched = m3gpuLaunchHashJobs(jobs, large);
+        if (launched < 0)
+        {
+            return -launched;
+        }
+        s_launches += launched;
+    }
+    rc = m3gpuLaunchHash(s_batch.dviews, s_batch.dorder + large, count - large, s_batch.dhash);
     if (rc != M3GPU_OK)
     {
         return rc;
     }
-    s_launches += 1;
+    s_launches += large < count ? 1 : 0;
     rc = Check(cudaGetLastError(), "hash launch");
     if (rc == M3GPU_OK)
     {
