@@ -921,17 +921,22 @@ __device__ uint8_t m3HfEdgeFlags(const m3TerrainCtx& c, int32_t t)
 }
 
 // Window triangle t's contact with the convex (manifold.c:1640-1672),
-// in the heightfield's frame.
-__device__ void m3HfCollideTriangle(const m3TerrainCtx& c, const m3Vec3 tri[3],
-                                    m3TriManifoldDev* local)
+// in the heightfield's frame.  OTHER is the convex's shape type, or
+// M3_HF_ANY to read it: a kernel for one type holds that type's code
+// alone (with all three in it, a third of its issue slots waited for
+// instructions).
+#define M3_HF_ANY (-1)
+template <int OTHER>
+__device__ __noinline__ void m3HfCollideTriangle(const m3TerrainCtx& c, const m3Vec3 tri[3],
+                                                 m3TriManifoldDev* local)
 {
     memset(local, 0, sizeof(*local));
-    if (c.otherType == M3_SHAPE_SPHERE)
+    if (OTHER == M3_SHAPE_SPHERE || (OTHER == M3_HF_ANY && c.otherType == M3_SHAPE_SPHERE))
     {
         m3SphereTriangleDev(local, c.s1, c.radius, tri);
         return;
     }
-    if (c.otherType == M3_SHAPE_CAPSULE)
+    if (OTHER == M3_SHAPE_CAPSULE || (OTHER == M3_HF_ANY && c.otherType == M3_SHAPE_CAPSULE))
     {
         m3CapsuleTriangleDev(local, c.s1, c.s2, c.radius, tri);
         return;
@@ -998,16 +1003,28 @@ __device__ __forceinline__ bool m3HfClaimEdge(m3HfClaims* set, int32_t wx, int32
     return m3HfClaimBit(set->edges, 4 * lo + code);
 }
 
-// Heightfield versus sphere, capsule or hull (manifold.c:1924-2071 and
-// the core it feeds, :1513-1906).  `fresh` arrives empty.
-__device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t hfShape,
-                                                 int32_t otherShape, bool hfIsA,
-                                                 m3Manifold* fresh)
+// The pair's context, the convex's bounds in the heightfield's frame and
+// the cell window; false when the convex is off the grid.  GROUP lanes
+// (a power of two; 1: each thread for itself) share the hull's vertices;
+// every lane of the warp takes part.
+struct m3TerrainPair
+{
+    m3TerrainCtx c;
+    m3Transform xfH;
+    m3Vec3 boundLo;
+    m3Vec3 boundHi;
+    m3real reach;
+    int32_t triCount;
+};
+
+template <int GROUP>
+__device__ __forceinline__ bool m3TerrainPairOf(const m3WorldView& w, int32_t hfShape,
+                                                int32_t otherShape, m3TerrainPair* out)
 {
     const m3HeightFieldDev hf = w.hfs[w.hfIndex[hfShape]];
     const m3Transform xfH = m3ShapeXf(w, hfShape);
     const m3Transform xfO = m3ShapeXf(w, otherShape);
-    m3TerrainCtx c;
+    m3TerrainCtx& c = out->c;
     c.heights = w.hfSamples + hf.sampleStart;
     c.nx = hf.nx;
     c.cell = hf.cellSize;
@@ -1034,7 +1051,45 @@ __device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t h
         c.pHull = m3Neg3(m3InvRotateVec3(c.qRel, c.pRel));
         boundLo = v3(3.4e38f, 3.4e38f, 3.4e38f);
         boundHi = v3(-3.4e38f, -3.4e38f, -3.4e38f);
-        for (int32_t v = 0; v < c.hull->vertexCount; ++v)
+        int32_t v = 0;
+        if (GROUP > 1)
+        {
+            bool finite = true;
+            for (int32_t u = threadIdx.x & (GROUP - 1); u < c.hull->vertexCount; u += GROUP)
+            {
+                const m3Vec3 p = m3Add3(m3RotateVec3(c.qRel, c.hull->vertices[u]), c.pRel);
+                finite = finite && p.x == p.x && p.y == p.y && p.z == p.z;
+                boundLo.x = m3MinF(boundLo.x, p.x);
+                boundLo.y = m3MinF(boundLo.y, p.y);
+                boundLo.z = m3MinF(boundLo.z, p.z);
+                boundHi.x = m3MaxF(boundHi.x, p.x);
+                boundHi.y = m3MaxF(boundHi.y, p.y);
+                boundHi.z = m3MaxF(boundHi.z, p.z);
+            }
+            __syncwarp();
+            for (int32_t o = GROUP / 2; o > 0; o >>= 1)
+            {
+                boundLo.x = m3MinF(boundLo.x, __shfl_xor_sync(0xFFFFFFFFu, boundLo.x, o));
+                boundLo.y = m3MinF(boundLo.y, __shfl_xor_sync(0xFFFFFFFFu, boundLo.y, o));
+                boundLo.z = m3MinF(boundLo.z, __shfl_xor_sync(0xFFFFFFFFu, boundLo.z, o));
+                boundHi.x = m3MaxF(boundHi.x, __shfl_xor_sync(0xFFFFFFFFu, boundHi.x, o));
+                boundHi.y = m3MaxF(boundHi.y, __shfl_xor_sync(0xFFFFFFFFu, boundHi.y, o));
+                boundHi.z = m3MaxF(boundHi.z, __shfl_xor_sync(0xFFFFFFFFu, boundHi.z, o));
+            }
+            const uint32_t group = (GROUP == 32 ? 0xFFFFFFFFu : (1u << (GROUP & 31)) - 1u)
+                                   << (threadIdx.x & 31 & ~(GROUP - 1));
+            if ((__ballot_sync(0xFFFFFFFFu, finite) & group) == group)
+            {
+                v = c.hull->vertexCount;
+            }
+            else
+            {
+                // Bounds over NaNs depend on the vertices' order.
+                boundLo = v3(3.4e38f, 3.4e38f, 3.4e38f);
+                boundHi = v3(-3.4e38f, -3.4e38f, -3.4e38f);
+            }
+        }
+        for (; v < c.hull->vertexCount; ++v)
         {
             const m3Vec3 p = m3Add3(m3RotateVec3(c.qRel, c.hull->vertices[v]), c.pRel);
             boundLo.x = m3MinF(boundLo.x, p.x);
@@ -1075,7 +1130,7 @@ __device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t h
     cz1 = cz1 > hf.nz - 2 ? hf.nz - 2 : cz1;
     if (cx1 < cx0 || cz1 < cz0)
     {
-        return; // off the grid
+        return false; // off the grid
     }
     if (cx1 - cx0 + 1 > M3_HF_WINDOW)
     {
@@ -1089,7 +1144,236 @@ __device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t h
     c.cz0 = cz0;
     c.wx = cx1 - cx0 + 2;
     c.wz = cz1 - cz0 + 2;
-    const int32_t triCount = 2 * (c.wx - 1) * (c.wz - 1);
+    out->xfH = xfH;
+    out->boundLo = boundLo;
+    out->boundHi = boundHi;
+    out->reach = reach;
+    out->triCount = 2 * (c.wx - 1) * (c.wz - 1);
+    return true;
+}
+
+// Whether window triangle `tri` comes near the convex's bounds.
+__device__ __forceinline__ bool m3HfNear(const m3TerrainPair& pair, const m3Vec3 tri[3])
+{
+    const m3real reach = pair.reach;
+    const m3real lox = m3MinF(tri[0].x, m3MinF(tri[1].x, tri[2].x)) - reach;
+    const m3real hix = m3MaxF(tri[0].x, m3MaxF(tri[1].x, tri[2].x)) + reach;
+    const m3real loy = m3MinF(tri[0].y, m3MinF(tri[1].y, tri[2].y)) - reach;
+    const m3real hiy = m3MaxF(tri[0].y, m3MaxF(tri[1].y, tri[2].y)) + reach;
+    const m3real loz = m3MinF(tri[0].z, m3MinF(tri[1].z, tri[2].z)) - reach;
+    const m3real hiz = m3MaxF(tri[0].z, m3MaxF(tri[1].z, tri[2].z)) + reach;
+    return !(pair.boundHi.x < lox || pair.boundLo.x > hix || pair.boundHi.y < loy ||
+             pair.boundLo.y > hiy || pair.boundHi.z < loz || pair.boundLo.z > hiz);
+}
+
+// Triangle t's contact as a candidate; whether it is accepted at once (a
+// face contact) or tentative.
+__device__ __forceinline__ bool m3HfCandidateOf(const m3TriManifoldDev& local, int32_t t,
+                                                m3HfCandidate* out)
+{
+    m3HfCandidate cand;
+    cand.dist2 = local.dist2;
+    cand.minSep = 3.4e38f;
+    for (int32_t k = 0; k < local.pointCount; ++k)
+    {
+        cand.minSep = m3MinF(cand.minSep, local.separation[k]);
+    }
+    cand.tri = (uint16_t)t;
+    cand.feature = (uint8_t)local.feature;
+    cand.pad = 0;
+    *out = cand;
+    if (local.feature == M3_TRI_FEATURE_HULL_FACE)
+    {
+        const m3real cosAngle = m3Dot3(local.triNormal, local.normal);
+        return cosAngle > 0.5f || cand.minSep < -2.0f * 0.005f;
+    }
+    return local.feature == 7;
+}
+
+// The deepest four of a cluster's points by (separation, id), sorted so,
+// of the first 2 x M3_MESH_CANDIDATE_CAP that come.
+struct m3HfKept
+{
+    m3Vec3 point[4];
+    m3real sep[4];
+    uint16_t id[4];
+    int32_t count;
+    int32_t seen;
+};
+
+__device__ __forceinline__ void m3HfKeep(m3HfKept* k, m3Vec3 point, m3real sep, uint16_t id)
+{
+    k->seen += 1;
+    int32_t at = k->count;
+    while (at > 0 && (sep < k->sep[at - 1] || (sep == k->sep[at - 1] && id < k->id[at - 1])))
+    {
+        at -= 1;
+    }
+    if (at >= 4)
+    {
+        return;
+    }
+    const int32_t last = k->count < 4 ? k->count : 3;
+    for (int32_t j = last; j > at; --j)
+    {
+        k->point[j] = k->point[j - 1];
+        k->sep[j] = k->sep[j - 1];
+        k->id[j] = k->id[j - 1];
+    }
+    k->point[at] = point;
+    k->sep[at] = sep;
+    k->id[at] = id;
+    k->count = k->count < 4 ? k->count + 1 : 4;
+}
+
+// The kept points in ascending id (the canonical point order), each split
+// into both anchors along the normal.
+__device__ __forceinline__ void m3HfEmit(const m3WorldView& w, const m3Transform& xfH,
+                                         int32_t hfShape, int32_t otherShape, bool hfIsA,
+                                         m3Vec3 repNormal, m3HfKept* kept, m3Manifold* fresh)
+{
+    for (int32_t a = 0; a < kept->count; ++a)
+    {
+        for (int32_t b = a + 1; b < kept->count; ++b)
+        {
+            if (kept->id[b] < kept->id[a])
+            {
+                const m3Vec3 tp = kept->point[a];
+                kept->point[a] = kept->point[b];
+                kept->point[b] = tp;
+                const m3real ts = kept->sep[a];
+                kept->sep[a] = kept->sep[b];
+                kept->sep[b] = ts;
+                const uint16_t ti = kept->id[a];
+                kept->id[a] = kept->id[b];
+                kept->id[b] = ti;
+            }
+        }
+    }
+    const int32_t meshBody = w.shapeBody[hfShape];
+    const int32_t otherBody = w.shapeBody[otherShape];
+    const m3Vec3 nWorld = m3RotateVec3(xfH.q, repNormal);
+    fresh->normal = hfIsA ? nWorld : m3Neg3(nWorld);
+    fresh->pointCount = kept->count;
+    for (int32_t k = 0; k < kept->count; ++k)
+    {
+        const m3Vec3 pw = m3RotateVec3(xfH.q, kept->point[k]);
+        const double px = xfH.p.x + (double)pw.x;
+        const double py = xfH.p.y + (double)pw.y;
+        const double pz = xfH.p.z + (double)pw.z;
+        const m3real half = 0.5f * kept->sep[k];
+        const m3Vec3 anchorMesh =
+            m3FromCom(w, meshBody, px - (double)(nWorld.x * half), py - (double)(nWorld.y * half),
+                      pz - (double)(nWorld.z * half));
+        const m3Vec3 anchorOther =
+            m3FromCom(w, otherBody, px + (double)(nWorld.x * half), py + (double)(nWorld.y * half),
+                      pz + (double)(nWorld.z * half));
+        fresh->points[k].anchorA = hfIsA ? anchorMesh : anchorOther;
+        fresh->points[k].anchorB = hfIsA ? anchorOther : anchorMesh;
+        fresh->points[k].separation = kept->sep[k];
+        fresh->points[k].id = kept->id[k];
+        fresh->points[k].flags = 0;
+    }
+}
+
+// Whether a tentative survives on an unclaimed feature, or on a real edge
+// (`convex`: its triangle's edge flags); claims its features.
+__device__ __forceinline__ bool m3HfSurvives(const m3TerrainCtx& c, const m3HfCandidate& cand,
+                                             uint8_t convex, m3HfClaims* set)
+{
+    int32_t idx[3];
+    m3HfTriangle(c, cand.tri, idx);
+    const bool newEdge1 = m3HfClaimEdge(set, c.wx, idx[0], idx[1]);
+    const bool newEdge2 = m3HfClaimEdge(set, c.wx, idx[1], idx[2]);
+    const bool newEdge3 = m3HfClaimEdge(set, c.wx, idx[2], idx[0]);
+    const bool newVert1 = m3HfClaimBit(set->verts, idx[0]);
+    const bool newVert2 = m3HfClaimBit(set->verts, idx[1]);
+    const bool newVert3 = m3HfClaimBit(set->verts, idx[2]);
+    switch (cand.feature)
+    {
+    case 1 | 2:
+        return (convex & 1) != 0 || newEdge1;
+    case 2 | 4:
+        return (convex & 2) != 0 || newEdge2;
+    case 1 | 4:
+        return (convex & 4) != 0 || newEdge3;
+    case 1:
+        return newVert1;
+    case 2:
+        return newVert2;
+    case 4:
+        return newVert3;
+    case M3_TRI_FEATURE_HULL_FACE:
+        return convex != 0 ||
+               (newEdge1 && newEdge2 && newEdge3 && newVert1 && newVert2 && newVert3);
+    default:
+        return false;
+    }
+}
+
+// A face contact claims its features.
+__device__ __forceinline__ void m3HfClaimFace(const m3TerrainCtx& c, const m3HfCandidate& cand,
+                                              m3HfClaims* set)
+{
+    int32_t idx[3];
+    m3HfTriangle(c, cand.tri, idx);
+    (void)m3HfClaimEdge(set, c.wx, idx[0], idx[1]);
+    (void)m3HfClaimEdge(set, c.wx, idx[1], idx[2]);
+    (void)m3HfClaimEdge(set, c.wx, idx[2], idx[0]);
+    (void)m3HfClaimBit(set->verts, idx[0]);
+    (void)m3HfClaimBit(set->verts, idx[1]);
+    (void)m3HfClaimBit(set->verts, idx[2]);
+}
+
+// One step of the reference's selection sort: the tentative of `from` and
+// behind with the least distance, ties to the lower triangle, to `from`.
+__device__ __forceinline__ void m3HfSelect(m3HfCandidate* tentative, int32_t from, int32_t count)
+{
+    int32_t best = from;
+    for (int32_t b = from + 1; b < count; ++b)
+    {
+        if (tentative[b].dist2 < tentative[best].dist2 ||
+            (tentative[b].dist2 == tentative[best].dist2 &&
+             tentative[b].tri < tentative[best].tri))
+        {
+            best = b;
+        }
+    }
+    const m3HfCandidate tmp = tentative[from];
+    tentative[from] = tentative[best];
+    tentative[best] = tmp;
+}
+
+// The deepest accepted contact, ties to the lower triangle
+// (manifold.c:1803-1818).
+__device__ __forceinline__ int32_t m3HfDeepest(const m3HfCandidate* accepted, int32_t count)
+{
+    int32_t repIndex = 0;
+    m3real repSep = 3.4e38f;
+    for (int32_t k = 0; k < count; ++k)
+    {
+        const m3real sep = accepted[k].minSep;
+        if (sep < repSep || (sep == repSep && accepted[k].tri < accepted[repIndex].tri))
+        {
+            repSep = sep;
+            repIndex = k;
+        }
+    }
+    return repIndex;
+}
+
+// Heightfield versus sphere, capsule or hull (manifold.c:1924-2071 and
+// the core it feeds, :1513-1906), by one thread.  `fresh` arrives empty.
+__device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t hfShape,
+                                                 int32_t otherShape, bool hfIsA,
+                                                 m3Manifold* fresh)
+{
+    m3TerrainPair pair;
+    if (!m3TerrainPairOf<1>(w, hfShape, otherShape, &pair))
+    {
+        return;
+    }
+    const m3TerrainCtx& c = pair.c;
 
     // Every window triangle in ascending order: face contacts accepted
     // at once, the rest tentative (manifold.c:1604-1703).
@@ -1098,55 +1382,27 @@ __device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t h
     m3HfCandidate tentative[M3_MESH_CANDIDATE_CAP];
     int32_t tentativeCount = 0;
     m3TriManifoldDev local;
-    for (int32_t t = 0; t < triCount; ++t)
+    m3Vec3 tri[3];
+    for (int32_t t = 0; t < pair.triCount; ++t)
     {
         if (faceCount >= M3_MESH_CANDIDATE_CAP || tentativeCount >= M3_MESH_CANDIDATE_CAP)
         {
             break;
         }
-        m3Vec3 tri[3];
         m3HfTriangleVerts(c, t, tri);
-        const m3real lox = m3MinF(tri[0].x, m3MinF(tri[1].x, tri[2].x)) - reach;
-        const m3real hix = m3MaxF(tri[0].x, m3MaxF(tri[1].x, tri[2].x)) + reach;
-        const m3real loy = m3MinF(tri[0].y, m3MinF(tri[1].y, tri[2].y)) - reach;
-        const m3real hiy = m3MaxF(tri[0].y, m3MaxF(tri[1].y, tri[2].y)) + reach;
-        const m3real loz = m3MinF(tri[0].z, m3MinF(tri[1].z, tri[2].z)) - reach;
-        const m3real hiz = m3MaxF(tri[0].z, m3MaxF(tri[1].z, tri[2].z)) + reach;
-        if (boundHi.x < lox || boundLo.x > hix || boundHi.y < loy || boundLo.y > hiy ||
-            boundHi.z < loz || boundLo.z > hiz)
+        if (!m3HfNear(pair, tri))
         {
             continue;
         }
-        m3HfCollideTriangle(c, tri, &local);
+        m3HfCollideTriangle<M3_HF_ANY>(c, tri, &local);
         if (local.pointCount == 0)
         {
             continue;
         }
         m3HfCandidate cand;
-        cand.dist2 = local.dist2;
-        cand.minSep = 3.4e38f;
-        for (int32_t k = 0; k < local.pointCount; ++k)
-        {
-            cand.minSep = m3MinF(cand.minSep, local.separation[k]);
-        }
-        cand.tri = (uint16_t)t;
-        cand.feature = (uint8_t)local.feature;
-        cand.pad = 0;
-        if (local.feature == 7)
+        if (m3HfCandidateOf(local, t, &cand))
         {
             faceAccepted[faceCount++] = cand;
-        }
-        else if (local.feature == M3_TRI_FEATURE_HULL_FACE)
-        {
-            const m3real cosAngle = m3Dot3(local.triNormal, local.normal);
-            if (cosAngle > 0.5f || cand.minSep < -2.0f * 0.005f)
-            {
-                faceAccepted[faceCount++] = cand;
-            }
-            else
-            {
-                tentative[tentativeCount++] = cand;
-            }
         }
         else
         {
@@ -1154,82 +1410,22 @@ __device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t h
         }
     }
 
-    // Face contacts claim their features first, in triangle order.
+    // Face contacts claim their features first, in triangle order; then
+    // the tentatives by ascending distance (the reference's selection
+    // sort, step for step).
     m3HfClaims set;
     memset(&set, 0, sizeof(set));
     for (int32_t k = 0; k < faceCount; ++k)
     {
-        int32_t idx[3];
-        m3HfTriangle(c, faceAccepted[k].tri, idx);
-        (void)m3HfClaimEdge(&set, c.wx, idx[0], idx[1]);
-        (void)m3HfClaimEdge(&set, c.wx, idx[1], idx[2]);
-        (void)m3HfClaimEdge(&set, c.wx, idx[2], idx[0]);
-        (void)m3HfClaimBit(set.verts, idx[0]);
-        (void)m3HfClaimBit(set.verts, idx[1]);
-        (void)m3HfClaimBit(set.verts, idx[2]);
+        m3HfClaimFace(c, faceAccepted[k], &set);
     }
-
-    // Tentatives by ascending distance, ties to the lower triangle (the
-    // reference's selection sort, step for step).
-    for (int32_t a = 0; a < tentativeCount; ++a)
+    for (int32_t k = 0; k < tentativeCount; ++k)
     {
-        int32_t best = a;
-        for (int32_t b = a + 1; b < tentativeCount; ++b)
-        {
-            if (tentative[b].dist2 < tentative[best].dist2 ||
-                (tentative[b].dist2 == tentative[best].dist2 &&
-                 tentative[b].tri < tentative[best].tri))
-            {
-                best = b;
-            }
-        }
-        const m3HfCandidate tmp = tentative[a];
-        tentative[a] = tentative[best];
-        tentative[best] = tmp;
+        m3HfSelect(tentative, k, tentativeCount);
     }
-
-    // A tentative survives on an unclaimed feature, or on a real edge.
     for (int32_t k = 0; k < tentativeCount && faceCount < M3_MESH_CANDIDATE_CAP; ++k)
     {
-        const int32_t t = tentative[k].tri;
-        int32_t idx[3];
-        m3HfTriangle(c, t, idx);
-        const bool newEdge1 = m3HfClaimEdge(&set, c.wx, idx[0], idx[1]);
-        const bool newEdge2 = m3HfClaimEdge(&set, c.wx, idx[1], idx[2]);
-        const bool newEdge3 = m3HfClaimEdge(&set, c.wx, idx[2], idx[0]);
-        const bool newVert1 = m3HfClaimBit(set.verts, idx[0]);
-        const bool newVert2 = m3HfClaimBit(set.verts, idx[1]);
-        const bool newVert3 = m3HfClaimBit(set.verts, idx[2]);
-        const uint8_t convex = m3HfEdgeFlags(c, t);
-        bool shouldCollide = false;
-        switch (tentative[k].feature)
-        {
-        case 1 | 2:
-            shouldCollide = (convex & 1) != 0 || newEdge1;
-            break;
-        case 2 | 4:
-            shouldCollide = (convex & 2) != 0 || newEdge2;
-            break;
-        case 1 | 4:
-            shouldCollide = (convex & 4) != 0 || newEdge3;
-            break;
-        case 1:
-            shouldCollide = newVert1;
-            break;
-        case 2:
-            shouldCollide = newVert2;
-            break;
-        case 4:
-            shouldCollide = newVert3;
-            break;
-        case M3_TRI_FEATURE_HULL_FACE:
-            shouldCollide = convex != 0 ||
-                            (newEdge1 && newEdge2 && newEdge3 && newVert1 && newVert2 && newVert3);
-            break;
-        default:
-            break;
-        }
-        if (shouldCollide)
+        if (m3HfSurvives(c, tentative[k], m3HfEdgeFlags(c, tentative[k].tri), &set))
         {
             faceAccepted[faceCount++] = tentative[k];
         }
@@ -1239,112 +1435,405 @@ __device__ __noinline__ void m3CollideTerrainDev(const m3WorldView& w, int32_t h
         return;
     }
 
-    // The deepest accepted contact (ties to the lower triangle) sets the
-    // cluster's normal (manifold.c:1803-1818).
-    int32_t repIndex = 0;
-    m3real repSep = 3.4e38f;
-    for (int32_t k = 0; k < faceCount; ++k)
-    {
-        const m3real sep = faceAccepted[k].minSep;
-        if (sep < repSep ||
-            (sep == repSep && faceAccepted[k].tri < faceAccepted[repIndex].tri))
-        {
-            repSep = sep;
-            repIndex = k;
-        }
-    }
-    m3Vec3 tri[3];
-    m3HfTriangleVerts(c, faceAccepted[repIndex].tri, tri);
-    m3HfCollideTriangle(c, tri, &local);
+    // The deepest accepted contact sets the cluster's normal; the
+    // cluster's points stream through.
+    m3HfTriangleVerts(c, faceAccepted[m3HfDeepest(faceAccepted, faceCount)].tri, tri);
+    m3HfCollideTriangle<M3_HF_ANY>(c, tri, &local);
     const m3Vec3 repNormal = local.normal;
-
-    // The cluster's points stream through; the deepest four by
-    // (separation, id) stay, sorted by (separation, id).
-    m3Vec3 keptPoint[4];
-    m3real keptSep[4];
-    uint16_t keptId[4];
-    int32_t keptCount = 0;
-    int32_t gCount = 0;
-    for (int32_t k = 0; k < faceCount && gCount < 2 * M3_MESH_CANDIDATE_CAP; ++k)
+    m3HfKept kept;
+    kept.count = 0;
+    kept.seen = 0;
+    for (int32_t k = 0; k < faceCount && kept.seen < 2 * M3_MESH_CANDIDATE_CAP; ++k)
     {
         m3HfTriangleVerts(c, faceAccepted[k].tri, tri);
-        m3HfCollideTriangle(c, tri, &local);
+        m3HfCollideTriangle<M3_HF_ANY>(c, tri, &local);
         if (m3Dot3(local.normal, repNormal) < 0.99f)
         {
             continue;
         }
-        for (int32_t p = 0; p < local.pointCount && gCount < 2 * M3_MESH_CANDIDATE_CAP; ++p)
+        for (int32_t p = 0; p < local.pointCount && kept.seen < 2 * M3_MESH_CANDIDATE_CAP; ++p)
         {
-            gCount += 1;
-            const m3real sep = local.separation[p];
-            const uint16_t id = (uint16_t)((faceAccepted[k].tri << 2) | local.localId[p]);
-            int32_t at = keptCount;
-            while (at > 0 && (sep < keptSep[at - 1] || (sep == keptSep[at - 1] && id < keptId[at - 1])))
-            {
-                at -= 1;
-            }
-            if (at >= 4)
-            {
-                continue;
-            }
-            const int32_t last = keptCount < 4 ? keptCount : 3;
-            for (int32_t j = last; j > at; --j)
-            {
-                keptPoint[j] = keptPoint[j - 1];
-                keptSep[j] = keptSep[j - 1];
-                keptId[j] = keptId[j - 1];
-            }
-            keptPoint[at] = local.point[p];
-            keptSep[at] = sep;
-            keptId[at] = id;
-            keptCount = keptCount < 4 ? keptCount + 1 : 4;
+            m3HfKeep(&kept, local.point[p], local.separation[p],
+                     (uint16_t)((faceAccepted[k].tri << 2) | local.localId[p]));
         }
     }
-    // Ascending id (the canonical point order).
-    for (int32_t a = 0; a < keptCount; ++a)
-    {
-        for (int32_t b = a + 1; b < keptCount; ++b)
-        {
-            if (keptId[b] < keptId[a])
-            {
-                const m3Vec3 tp = keptPoint[a];
-                keptPoint[a] = keptPoint[b];
-                keptPoint[b] = tp;
-                const m3real ts = keptSep[a];
-                keptSep[a] = keptSep[b];
-                keptSep[b] = ts;
-                const uint16_t ti = keptId[a];
-                keptId[a] = keptId[b];
-                keptId[b] = ti;
-            }
-        }
-    }
+    m3HfEmit(w, pair.xfH, hfShape, otherShape, hfIsA, repNormal, &kept, fresh);
+}
 
-    // Emit: each point splits into both anchors along the normal.
-    const int32_t meshBody = w.shapeBody[hfShape];
-    const int32_t otherBody = w.shapeBody[otherShape];
-    const m3Vec3 nWorld = m3RotateVec3(xfH.q, repNormal);
-    fresh->normal = hfIsA ? nWorld : m3Neg3(nWorld);
-    fresh->pointCount = keptCount;
-    for (int32_t k = 0; k < keptCount; ++k)
+// Triangles' contacts in shared memory: normals, and points with their
+// separations and ids.
+struct m3TerrainContacts
+{
+    float4 point[32][4];
+    m3Vec3 normal[32];
+    uint16_t id[32][4];
+    uint8_t points[32];
+};
+
+__device__ __forceinline__ void m3TerrainKeepContact(m3TerrainContacts* s, int32_t at, int32_t t,
+                                                     const m3TriManifoldDev& local)
+{
+    s->normal[at] = local.normal;
+    s->points[at] = (uint8_t)local.pointCount;
+    for (int32_t p = 0; p < local.pointCount; ++p)
     {
-        const m3Vec3 pw = m3RotateVec3(xfH.q, keptPoint[k]);
-        const double px = xfH.p.x + (double)pw.x;
-        const double py = xfH.p.y + (double)pw.y;
-        const double pz = xfH.p.z + (double)pw.z;
-        const m3real half = 0.5f * keptSep[k];
-        const m3Vec3 anchorMesh =
-            m3FromCom(w, meshBody, px - (double)(nWorld.x * half), py - (double)(nWorld.y * half),
-                      pz - (double)(nWorld.z * half));
-        const m3Vec3 anchorOther =
-            m3FromCom(w, otherBody, px + (double)(nWorld.x * half), py + (double)(nWorld.y * half),
-                      pz + (double)(nWorld.z * half));
-        fresh->points[k].anchorA = hfIsA ? anchorMesh : anchorOther;
-        fresh->points[k].anchorB = hfIsA ? anchorOther : anchorMesh;
-        fresh->points[k].separation = keptSep[k];
-        fresh->points[k].id = keptId[k];
-        fresh->points[k].flags = 0;
+        s->point[at][p] = make_float4(local.point[p].x, local.point[p].y, local.point[p].z,
+                                      local.separation[p]);
+        s->id[at][p] = (uint16_t)((t << 2) | local.localId[p]);
     }
+}
+
+// One accepted contact's points into the kept ones, when it belongs to the
+// cluster.
+__device__ __forceinline__ void m3HfKeepContact(const m3TerrainContacts& s, int32_t at,
+                                                m3Vec3 repNormal, m3HfKept* kept)
+{
+    if (m3Dot3(s.normal[at], repNormal) < 0.99f)
+    {
+        return;
+    }
+    for (int32_t p = 0; p < s.points[at] && kept->seen < 2 * M3_MESH_CANDIDATE_CAP; ++p)
+    {
+        const float4 q = s.point[at][p];
+        m3HfKeep(kept, v3(q.x, q.y, q.z), q.w, s.id[at][p]);
+    }
+}
+
+// The same by one warp, a triangle a lane: the pairs with many near
+// triangles of a kernel that gives the others a group of lanes.  The lanes
+// collide the near triangles side by side (the edge flags of the
+// tentatives too), and lane `leader` makes the short ordered parts (the
+// selection, the claims, the clustering) and has the result.
+struct m3TerrainWarp
+{
+    m3TerrainContacts contacts;
+    m3HfCandidate accepted[M3_MESH_CANDIDATE_CAP];
+    m3HfCandidate tentative[M3_MESH_CANDIDATE_CAP];
+    uint8_t convex[M3_MESH_CANDIDATE_CAP];
+    m3HfClaims set;
+    uint16_t near[2 * M3_HF_WINDOW * M3_HF_WINDOW];
+    int32_t acceptedCount;
+};
+
+template <int OTHER>
+__device__ __noinline__ void m3CollideTerrainWarp(const m3WorldView& w, int32_t hfShape,
+                                                  int32_t otherShape, bool hfIsA,
+                                                  m3TerrainWarp* s, int32_t leader,
+                                                  m3Manifold* fresh)
+{
+    const int32_t lane = threadIdx.x & 31;
+    const uint32_t before = (1u << lane) - 1u;
+    m3TerrainPair pair;
+    if (!m3TerrainPairOf<32>(w, hfShape, otherShape, &pair))
+    {
+        return;
+    }
+    const m3TerrainCtx& c = pair.c;
+    __syncwarp();
+    int32_t nearCount = 0;
+    for (int32_t t0 = 0; t0 < pair.triCount; t0 += 32)
+    {
+        const int32_t t = t0 + lane;
+        bool near = false;
+        if (t < pair.triCount)
+        {
+            m3Vec3 tri[3];
+            m3HfTriangleVerts(c, t, tri);
+            near = m3HfNear(pair, tri);
+        }
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, near);
+        if (near)
+        {
+            s->near[nearCount + __popc(mask & before)] = (uint16_t)t;
+        }
+        nearCount += __popc(mask);
+    }
+    __syncwarp();
+    int32_t faceCount = 0;
+    int32_t tentativeCount = 0;
+    m3TriManifoldDev local;
+    m3Vec3 tri[3];
+    for (int32_t n0 = 0; n0 < nearCount; n0 += 32)
+    {
+        const int32_t n = n0 + lane;
+        const int32_t t = n < nearCount ? s->near[n] : 0;
+        m3HfCandidate cand;
+        bool face = false;
+        bool any = false;
+        if (n < nearCount)
+        {
+            m3HfTriangleVerts(c, t, tri);
+            m3HfCollideTriangle<OTHER>(c, tri, &local);
+            any = local.pointCount != 0;
+            face = any && m3HfCandidateOf(local, t, &cand);
+        }
+        // In triangle order; the walk ends before the first triangle that
+        // finds either list full.
+        const uint32_t faces = __ballot_sync(0xFFFFFFFFu, face);
+        const uint32_t others = __ballot_sync(0xFFFFFFFFu, any && !face);
+        const int32_t f = faceCount + __popc(faces & before);
+        const int32_t o = tentativeCount + __popc(others & before);
+        const bool in = f < M3_MESH_CANDIDATE_CAP && o < M3_MESH_CANDIDATE_CAP;
+        if (any && in)
+        {
+            if (face)
+            {
+                s->accepted[f] = cand;
+            }
+            else
+            {
+                s->tentative[o] = cand;
+            }
+        }
+        const uint32_t ins = __ballot_sync(0xFFFFFFFFu, in);
+        faceCount += __popc(faces & ins);
+        tentativeCount += __popc(others & ins);
+        if (ins != 0xFFFFFFFFu || faceCount >= M3_MESH_CANDIDATE_CAP ||
+            tentativeCount >= M3_MESH_CANDIDATE_CAP)
+        {
+            break;
+        }
+    }
+    for (int32_t i = lane; i < (int32_t)(sizeof(m3HfClaims) / 4); i += 32)
+    {
+        ((uint32_t*)&s->set)[i] = 0u;
+    }
+    __syncwarp();
+    for (int32_t k = lane; k < tentativeCount; k += 32)
+    {
+        s->convex[k] = m3HfEdgeFlags(c, s->tentative[k].tri);
+    }
+    __syncwarp();
+    if (lane == leader)
+    {
+        for (int32_t k = 0; k < faceCount; ++k)
+        {
+            m3HfClaimFace(c, s->accepted[k], &s->set);
+        }
+        // The candidates' spare byte carries their place in the unsorted
+        // list through the selection: their edge flags'.
+        for (int32_t k = 0; k < tentativeCount; ++k)
+        {
+            s->tentative[k].pad = (uint8_t)k;
+        }
+        for (int32_t k = 0; k < tentativeCount; ++k)
+        {
+            m3HfSelect(s->tentative, k, tentativeCount);
+        }
+        int32_t count = faceCount;
+        for (int32_t k = 0; k < tentativeCount && count < M3_MESH_CANDIDATE_CAP; ++k)
+        {
+            const m3HfCandidate cand = s->tentative[k];
+            if (m3HfSurvives(c, cand, s->convex[cand.pad], &s->set))
+            {
+                s->accepted[count++] = cand;
+            }
+        }
+        s->acceptedCount = count;
+    }
+    __syncwarp();
+    const int32_t accepted = s->acceptedCount;
+    if (accepted == 0)
+    {
+        return;
+    }
+    const int32_t rep = m3HfDeepest(s->accepted, accepted);
+    m3HfKept kept;
+    kept.count = 0;
+    kept.seen = 0;
+    m3HfTriangleVerts(c, s->accepted[rep].tri, tri);
+    m3HfCollideTriangle<OTHER>(c, tri, &local);
+    const m3Vec3 repNormal = local.normal;
+    for (int32_t k0 = 0; k0 < accepted; k0 += 32)
+    {
+        const int32_t mine = k0 + lane;
+        __syncwarp();
+        if (mine < accepted)
+        {
+            m3HfTriangleVerts(c, s->accepted[mine].tri, tri);
+            m3HfCollideTriangle<OTHER>(c, tri, &local);
+            m3TerrainKeepContact(&s->contacts, lane, s->accepted[mine].tri, local);
+        }
+        __syncwarp();
+        if (lane != leader)
+        {
+            continue;
+        }
+        for (int32_t k = k0; k < k0 + 32 && k < accepted && kept.seen < 2 * M3_MESH_CANDIDATE_CAP;
+             ++k)
+        {
+            m3HfKeepContact(s->contacts, k - k0, repNormal, &kept);
+        }
+    }
+    if (lane == leader)
+    {
+        m3HfEmit(w, pair.xfH, hfShape, otherShape, hfIsA, repNormal, &kept, fresh);
+    }
+}
+
+
+// The same by GROUP lanes, 32 / GROUP pairs a warp: a thread that walked a
+// window of 30 to 50 triangles by itself made the heightfield-hull kernel a
+// tail of 1.27 ms on 256 worlds of 32 to 512 bodies, and a whole warp a
+// pair had 5.5 of its 32 lanes at work.  The group collides its near
+// triangles side by side and keeps the contacts in shared memory; its
+// first lane makes the ordered parts beside the other groups' first
+// lanes.  False when more than M3_HF_GROUP_NEAR triangles are near (the
+// caller gives the pair a warp).  `pairIn`: whether the group has a pair;
+// every lane of the warp calls.
+#define M3_HF_GROUP_NEAR 32
+struct m3TerrainGroup
+{
+    m3TerrainContacts contacts;
+    m3HfCandidate cand[M3_HF_GROUP_NEAR];
+    m3HfClaims set;
+    uint16_t near[M3_HF_GROUP_NEAR];
+    uint8_t kind[M3_HF_GROUP_NEAR]; // of a near triangle's contact: none, face, tentative
+    uint8_t convex[M3_HF_GROUP_NEAR];
+    uint8_t order[M3_HF_GROUP_NEAR];
+};
+
+template <int OTHER, int GROUP>
+__device__ __forceinline__ bool m3CollideTerrainGroup(const m3WorldView& w, int32_t hfShape,
+                                                      int32_t otherShape, bool hfIsA, bool pairIn,
+                                                      m3TerrainGroup* s, m3Manifold* fresh)
+{
+    const int32_t sub = threadIdx.x & (GROUP - 1);
+    const int32_t shift = threadIdx.x & 31 & ~(GROUP - 1);
+    const uint32_t below = (1u << sub) - 1u;
+    const uint32_t members = (1u << GROUP) - 1u;
+    m3TerrainPair pair;
+    pair.triCount = 0;
+    if (!m3TerrainPairOf<GROUP>(w, hfShape, otherShape, &pair) || !pairIn)
+    {
+        pair.triCount = 0;
+    }
+    const m3TerrainCtx& c = pair.c;
+    __syncwarp();
+    m3Vec3 tri[3];
+    int32_t nearCount = 0;
+    for (int32_t t0 = 0; __any_sync(0xFFFFFFFFu, t0 < pair.triCount); t0 += GROUP)
+    {
+        const int32_t t = t0 + sub;
+        bool near = false;
+        if (t < pair.triCount)
+        {
+            m3HfTriangleVerts(c, t, tri);
+            near = m3HfNear(pair, tri);
+        }
+        const uint32_t mask = __ballot_sync(0xFFFFFFFFu, near) >> shift & members;
+        const int32_t at = nearCount + __popc(mask & below);
+        if (near && at < M3_HF_GROUP_NEAR)
+        {
+            s->near[at] = (uint16_t)t;
+        }
+        nearCount += __popc(mask);
+    }
+    const bool fits = nearCount <= M3_HF_GROUP_NEAR;
+    nearCount = fits ? nearCount : 0;
+    for (int32_t i = sub; i < (int32_t)(sizeof(m3HfClaims) / 4); i += GROUP)
+    {
+        ((uint32_t*)&s->set)[i] = 0u;
+    }
+    __syncwarp();
+    for (int32_t n0 = 0; __any_sync(0xFFFFFFFFu, n0 < nearCount); n0 += GROUP)
+    {
+        const int32_t n = n0 + sub;
+        if (n < nearCount)
+        {
+            const int32_t t = s->near[n];
+            m3TriManifoldDev local;
+            m3HfTriangleVerts(c, t, tri);
+            m3HfCollideTriangle<OTHER>(c, tri, &local);
+            uint8_t kind = 0;
+            if (local.pointCount != 0)
+            {
+                m3HfCandidate cand;
+                kind = m3HfCandidateOf(local, t, &cand) ? 1 : 2;
+                s->cand[n] = cand;
+                m3TerrainKeepContact(&s->contacts, n, t, local);
+                if (kind == 2)
+                {
+                    s->convex[n] = m3HfEdgeFlags(c, t);
+                }
+            }
+            s->kind[n] = kind;
+        }
+        __syncwarp();
+    }
+    if (sub == 0 && nearCount > 0)
+    {
+        // Face contacts first, in triangle order, then the tentatives by
+        // ascending distance (the reference's selection sort, step for
+        // step) that survive.
+        int32_t accepted = 0;
+        for (int32_t n = 0; n < nearCount; ++n)
+        {
+            if (s->kind[n] == 1)
+            {
+                m3HfClaimFace(c, s->cand[n], &s->set);
+                s->order[accepted++] = (uint8_t)n;
+            }
+        }
+        int32_t listed = accepted;
+        for (int32_t n = 0; n < nearCount; ++n)
+        {
+            if (s->kind[n] == 2)
+            {
+                s->order[listed++] = (uint8_t)n;
+            }
+        }
+        for (int32_t k = accepted; k < listed; ++k)
+        {
+            int32_t best = k;
+            for (int32_t b = k + 1; b < listed; ++b)
+            {
+                const m3HfCandidate& x = s->cand[s->order[b]];
+                const m3HfCandidate& y = s->cand[s->order[best]];
+                if (x.dist2 < y.dist2 || (x.dist2 == y.dist2 && x.tri < y.tri))
+                {
+                    best = b;
+                }
+            }
+            const uint8_t n = s->order[best];
+            s->order[best] = s->order[k];
+            s->order[k] = n;
+        }
+        for (int32_t k = accepted; k < listed; ++k)
+        {
+            const uint8_t n = s->order[k];
+            if (m3HfSurvives(c, s->cand[n], s->convex[n], &s->set))
+            {
+                s->order[accepted++] = n;
+            }
+        }
+        if (accepted > 0)
+        {
+            int32_t rep = 0;
+            m3real repSep = 3.4e38f;
+            for (int32_t k = 0; k < accepted; ++k)
+            {
+                const m3HfCandidate& x = s->cand[s->order[k]];
+                if (x.minSep < repSep ||
+                    (x.minSep == repSep && x.tri < s->cand[s->order[rep]].tri))
+                {
+                    repSep = x.minSep;
+                    rep = k;
+                }
+            }
+            const m3Vec3 repNormal = s->contacts.normal[s->order[rep]];
+            m3HfKept kept;
+            kept.count = 0;
+            kept.seen = 0;
+            for (int32_t k = 0; k < accepted; ++k)
+            {
+                m3HfKeepContact(s->contacts, s->order[k], repNormal, &kept);
+            }
+            m3HfEmit(w, pair.xfH, hfShape, otherShape, hfIsA, repNormal, &kept, fresh);
+        }
+    }
+    __syncwarp();
+    return fits;
 }
 
 #endif // M3_TERRAIN_CUH

@@ -2089,6 +2089,81 @@ __global__ void __launch_bounds__(128)
     }
 }
 
+// The same for a heightfield family whose triangle kernel is long (capsule
+// or hull partners): a group of lanes a pair, and a warp for the pairs
+// with more near triangles than a group holds.  Groups of 8 took the 256
+// terrain worlds' narrowphase to 0.77 ms a step; of 4, 0.97, of 16, 1.2,
+// a warp a pair 1.9, a thread a pair 2.0.
+#define M3_TERRAIN_GROUP 8
+#define M3_TERRAIN_THREADS 64
+template <int F>
+__global__ void __launch_bounds__(M3_TERRAIN_THREADS)
+    m3NarrowTerrainKernel(const m3WorldView* views, const int32_t* offsets, int32_t count,
+                          const int32_t* famStart, const int32_t* bucket)
+{
+    constexpr int OTHER = F == M3F_TERRAIN_CAPSULE ? M3_SHAPE_CAPSULE : M3_SHAPE_HULL;
+    constexpr int32_t PAIRS = 32 / M3_TERRAIN_GROUP; // a warp
+    union Shared
+    {
+        m3TerrainGroup group[PAIRS];
+        m3TerrainWarp warp;
+    };
+    __shared__ __align__(16) uint8_t s_raw[M3_TERRAIN_THREADS / 32][sizeof(Shared)];
+    Shared& s = *(Shared*)s_raw[threadIdx.x >> 5];
+    const int32_t lane = threadIdx.x & 31;
+    const int32_t mine = lane / M3_TERRAIN_GROUP;
+    const int32_t start = famStart[F];
+    const int32_t pairs = famStart[F + 1] - start;
+    const int32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (int32_t p0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PAIRS; p0 < pairs;
+         p0 += warps * PAIRS)
+    {
+        // A group past the end goes along with the last pair.
+        const bool in = p0 + mine < pairs;
+        const int32_t g = bucket[start + (in ? p0 + mine : pairs - 1)];
+        const int32_t wi = FlatWorld(offsets, count, g);
+        const m3WorldView& w = views[wi];
+        const m3WorldScalars* sc = w.sc;
+        const int32_t k = g - offsets[wi];
+        const int32_t cur = sc->pairBuf;
+        const uint64_t* newKeys = cur == 0 ? w.keys1 : w.keys0;
+        const uint64_t key = newKeys[k];
+        const int32_t shapeA = (int32_t)(key >> 32);
+        const int32_t shapeB = (int32_t)(key & 0xFFFFFFFFu);
+        const int32_t hfShape = w.shapeType[shapeA] == M3_SHAPE_HEIGHTFIELD ? shapeA : shapeB;
+        const int32_t otherShape = hfShape == shapeA ? shapeB : shapeA;
+        m3Manifold fresh = m3EmptyManifold();
+        const bool fits = m3CollideTerrainGroup<OTHER, M3_TERRAIN_GROUP>(
+            w, hfShape, otherShape, hfShape == shapeA, in, &s.group[mine], &fresh);
+        uint32_t large = __ballot_sync(0xFFFFFFFFu, !fits && in);
+        while (large != 0)
+        {
+            const int32_t leader = __ffs((int)large) - 1;
+            large &= ~(((1u << M3_TERRAIN_GROUP) - 1u) << leader);
+            const m3WorldView& lw = views[__shfl_sync(0xFFFFFFFFu, wi, leader)];
+            const int32_t hf = __shfl_sync(0xFFFFFFFFu, hfShape, leader);
+            const int32_t other = __shfl_sync(0xFFFFFFFFu, otherShape, leader);
+            const bool first = __shfl_sync(0xFFFFFFFFu, (int32_t)(hfShape == shapeA), leader) != 0;
+            m3Manifold whole = m3EmptyManifold();
+            m3CollideTerrainWarp<OTHER>(lw, hf, other, first, &s.warp, leader, &whole);
+            if (lane == leader)
+            {
+                fresh = whole;
+            }
+            __syncwarp();
+        }
+        if (in && lane % M3_TERRAIN_GROUP == 0)
+        {
+            const uint64_t* oldKeys = cur == 0 ? w.keys0 : w.keys1;
+            const m3Manifold* oldMan = cur == 0 ? w.man0 : w.man1;
+            m3Manifold* newMan = cur == 0 ? w.man1 : w.man0;
+            m3WarmCarry(&fresh, key, oldKeys, oldMan, sc->pairCount, k);
+            newMan[k] = fresh;
+        }
+        __syncwarp();
+    }
+}
+
 // ---------------------------------------------------------------------
 // Islands (solver.c:3437-3578): a lock-free union-find whose links
 // always point a root at a smaller root, so each component's final
@@ -5359,16 +5434,26 @@ static int32_t s_narrowGrid = 148 * 16;
 // kernel per covered family over its bucket.
 #define M3_NARROW_LAUNCHES (2 + M3F_TERRAIN_SPHERE)
 #define M3_TERRAIN_LAUNCHES 3
-// Batches of at most this many worlds take the single narrowphase kernel.
+// Batches of at most this many worlds may take the single narrowphase kernel.
 #define M3_NARROW_SMALL_BATCH 4
 
-static void LaunchNarrow(const m3WorldView* views, const int32_t* offsets, int32_t count,
-                         bool terrain)
+// Whether a batch's pairs go through the single kernel: few worlds, at
+// most M3_NARROW_SMALL_SHAPES shape slots in all (3,001 bodies took 0.38 ms
+// a step in one kernel and 0.49 by families, 20,000 boxes 0.34 and 0.20)
+// and no heightfield (whose pairs need groups of lanes).
+#define M3_NARROW_SMALL_SHAPES 4095
+static bool NarrowInOne(int32_t count, int64_t shapes, bool terrain)
 {
-    if (count <= M3_NARROW_SMALL_BATCH)
+    return count <= M3_NARROW_SMALL_BATCH && shapes <= M3_NARROW_SMALL_SHAPES && !terrain;
+}
+
+static void LaunchNarrow(const m3WorldView* views, const int32_t* offsets, int32_t count,
+                         int64_t shapes, bool terrain)
+{
+    if (NarrowInOne(count, shapes, terrain))
     {
-        // A handful of worlds: one kernel over every family beats the
-        // bucketing's nine launches.
+        // A handful of small worlds: one kernel over every family beats
+        // the bucketing's nine launches.
         m3NarrowKernel<<<148, 128>>>(views, offsets, count);
         return;
     }
@@ -5379,28 +5464,45 @@ static void LaunchNarrow(const m3WorldView* views, const int32_t* offsets, int32
     m3FamilyScatterKernel<<<M3_FAMILY_BLOCKS, M3_FAMILY_THREADS>>>(views, offsets, count,
                                                                    blockHist, famStart,
                                                                    s_batch.dbucket);
-    m3NarrowFamilyKernel<M3F_PLANE_HULL>
-        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-    m3NarrowFamilyKernel<M3F_HULL_HULL>
-        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-    m3NarrowFamilyKernel<M3F_PLANE_CAPSULE>
-        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-    m3NarrowFamilyKernel<M3F_CAPSULE_HULL>
-        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-    m3NarrowFamilyKernel<M3F_ROUND><<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-    m3NarrowFamilyKernel<M3F_PLANE_SPHERE>
-        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-    m3NarrowFamilyKernel<M3F_SPHERE_SPHERE>
-        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
+    // The families side by side: each kernel is a tail of long pairs that
+    // leaves most issue slots free (one after another, the ten took 1.0 ms
+    // a step on 256 terrain worlds).
+    cudaEventRecord(s_classStreams.fork, 0);
+    for (int32_t c = 0; c < M3_CLASSES; ++c)
+    {
+        cudaStreamWaitEvent(s_classStreams.stream[c], s_classStreams.fork, 0);
+    }
+    const cudaStream_t s0 = s_classStreams.stream[0];
+    const cudaStream_t s1 = s_classStreams.stream[1];
+    const cudaStream_t s2 = s_classStreams.stream[2];
     if (terrain)
     {
         // Heightfield pairs, only in batches holding a heightfield.
+        m3NarrowTerrainKernel<M3F_TERRAIN_HULL>
+            <<<s_narrowGrid, M3_TERRAIN_THREADS, 0, s0>>>(views, offsets, count, famStart, bucket);
+        m3NarrowTerrainKernel<M3F_TERRAIN_CAPSULE>
+            <<<s_narrowGrid, M3_TERRAIN_THREADS, 0, s1>>>(views, offsets, count, famStart, bucket);
         m3NarrowFamilyKernel<M3F_TERRAIN_SPHERE>
-            <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-        m3NarrowFamilyKernel<M3F_TERRAIN_CAPSULE>
-            <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
-        m3NarrowFamilyKernel<M3F_TERRAIN_HULL>
-            <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
+            <<<s_narrowGrid, 128, 0, s2>>>(views, offsets, count, famStart, bucket);
+    }
+    m3NarrowFamilyKernel<M3F_HULL_HULL>
+        <<<s_narrowGrid, 128>>>(views, offsets, count, famStart, bucket);
+    m3NarrowFamilyKernel<M3F_CAPSULE_HULL>
+        <<<s_narrowGrid, 128, 0, s0>>>(views, offsets, count, famStart, bucket);
+    m3NarrowFamilyKernel<M3F_ROUND>
+        <<<s_narrowGrid, 128, 0, s1>>>(views, offsets, count, famStart, bucket);
+    m3NarrowFamilyKernel<M3F_PLANE_HULL>
+        <<<s_narrowGrid, 128, 0, s2>>>(views, offsets, count, famStart, bucket);
+    m3NarrowFamilyKernel<M3F_PLANE_CAPSULE>
+        <<<s_narrowGrid, 128, 0, s0>>>(views, offsets, count, famStart, bucket);
+    m3NarrowFamilyKernel<M3F_PLANE_SPHERE>
+        <<<s_narrowGrid, 128, 0, s1>>>(views, offsets, count, famStart, bucket);
+    m3NarrowFamilyKernel<M3F_SPHERE_SPHERE>
+        <<<s_narrowGrid, 128, 0, s2>>>(views, offsets, count, famStart, bucket);
+    for (int32_t c = 0; c < M3_CLASSES; ++c)
+    {
+        cudaEventRecord(s_classStreams.join[c], s_classStreams.stream[c]);
+        cudaStreamWaitEvent(0, s_classStreams.join[c], 0);
     }
 }
 
@@ -6127,9 +6229,11 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
     }
     const cudaStream_t treeStream = s_classStreams.tree;
     int32_t mostShapes = 1;
+    int64_t allShapes = 0;
     for (int32_t i = 0; i < count; ++i)
     {
         const int32_t shapes = worlds[i]->hv.sc->shapeMax;
+        allShapes += shapes;
         mostShapes = shapes > mostShapes ? shapes : mostShapes;
     }
     const int32_t sortCap = BroadSortCap(mostShapes);
@@ -6211,12 +6315,12 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
             }
         }
         m3PairOffsetsKernel<<<1, M3_BLOCK>>>(s_batch.dviews, count, s_batch.doffsets);
-        LaunchNarrow(s_batch.dviews, s_batch.doffsets, count, anyTerrain);
+        LaunchNarrow(s_batch.dviews, s_batch.doffsets, count, allShapes, anyTerrain);
         cudaEventRecord(ev[2]);
         LaunchSolve(s_batch.dviews, s_batch.dorder, count, dt, substeps, s_batch.cacheBytes,
                     ev + 3, s_batch.classFirst, s_batch.classCache, wideBlocks);
         cudaEventRecord(ev[5]);
-        s_launches += 5 + (count <= M3_NARROW_SMALL_BATCH ? 1 : M3_NARROW_LAUNCHES + (anyTerrain ? M3_TERRAIN_LAUNCHES : 0));
+        s_launches += 5 + (NarrowInOne(count, allShapes, anyTerrain) ? 1 : M3_NARROW_LAUNCHES + (anyTerrain ? M3_TERRAIN_LAUNCHES : 0));
     }
     // The trees catch up later: replays already launched finish on their
     // own stream, recorded steps not yet launched wait in the ring; a
