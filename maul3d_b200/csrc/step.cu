@@ -122,6 +122,7 @@ struct m3StepPlan
     int32_t moverCount;
     int32_t anyRestitution;
     int32_t levels; // joint/contact schedule levels; levelStart[levels] starts the overflow
+    int32_t islands; // a wide world: whether its substep loop runs by islands
     int32_t starts[M3_GRAPH_COLORS + 2]; // colour sizes (as offsets) of the colouring
 };
 
@@ -4289,8 +4290,10 @@ __global__ void __launch_bounds__(NT, 2) m3WideSubstepKernel(const m3WorldView* 
         }
         return true;
     };
-    // The substep loop (solver.c:4085-4203).
-    for (int32_t sub = 0; sub < substeps; ++sub)
+    // The substep loop (solver.c:4085-4203), unless m3IslandSubstepKernel
+    // has run it.
+    const int32_t loops = s.plan->islands != 0 ? 0 : substeps;
+    for (int32_t sub = 0; sub < loops; ++sub)
     {
         for (int32_t m = gtid; m < moverCount; m += gstride)
         {
@@ -4426,6 +4429,430 @@ __global__ void __launch_bounds__(NT, 2) m3WideSubstepKernel(const m3WorldView* 
     }
     M3_WIDE_MARK(M3_PHASE_STORE)
 #undef M3_WIDE_MARK
+}
+
+// ---------------------------------------------------------------------
+// A wide world by islands.  Bodies of different islands share no row, so a
+// block that owns whole islands runs their substep loop by itself: its
+// levels are separated by block barriers instead of grid barriers (8 to
+// 10 us each; 100 towers of joints, about 100 levels a pass, spent 26 ms a
+// step on 24 passes).  The islands (the wake pass's union-find) go to
+// groups, one a block, in root order by an even share of their work; the
+// rows keep their levels and are sorted by (group, level), so inside a
+// body every row keeps its place.  The groups are used when no group has
+// more than M3_ISLAND_ROWS of work a level (four rows a thread, about the
+// time of a grid barrier) and nothing moves but dynamic bodies (a
+// kinematic body's poses are read by several groups).  The tables lie in
+// the sweep's pair list, which is spent.
+// ---------------------------------------------------------------------
+#define M3_ISLAND_ROWS 1024
+#define M3_ISLAND_THREADS 256
+
+struct m3IslandTables
+{
+    int32_t* contact; // groups x (levels + 1) + 1 row starts, group-major
+    int32_t* joint;   // groups x jointLevels + 1
+    int32_t* mover;   // groups + 1
+    int32_t* contactFill;
+    int32_t* jointFill;
+    int32_t* moverFill;
+    int32_t contacts; // entries
+    int32_t joints;
+    bool fits;
+};
+
+__device__ __forceinline__ m3IslandTables IslandTables(const m3Scratch& s, int32_t pairCap,
+                                                       int32_t groups)
+{
+    m3IslandTables t;
+    t.contacts = groups * (s.plan->levels + 1);
+    t.joints = groups * s.plan->jointLevels;
+    int32_t* at = (int32_t*)s.sweepPairs;
+    t.contact = at;
+    t.joint = t.contact + t.contacts + 1;
+    t.mover = t.joint + t.joints + 1;
+    t.contactFill = t.mover + groups + 1;
+    t.jointFill = t.contactFill + t.contacts;
+    t.moverFill = t.jointFill + t.joints;
+    t.fits = (int64_t)(t.moverFill + groups - at) <= 2 * (int64_t)pairCap;
+    return t;
+}
+
+// The dynamic body that says which island a joint row belongs to.
+__device__ __forceinline__ int32_t JointIslandBody(const m3WorldView& w, int2 ab)
+{
+    return w.btype[ab.x] == M3_BODY_DYNAMIC && w.awake[ab.x] != 0 ? ab.x : ab.y;
+}
+
+// Clears the islands' work (per root, in s.forced).
+__global__ void __launch_bounds__(M3_BLOCK) m3IslandClearKernel(const m3WorldView* views,
+                                                               const int32_t* order)
+{
+    const m3WorldView& w = views[order[0]];
+    const m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    for (int32_t i = blockIdx.x * M3_BLOCK + threadIdx.x; i < sc->bodyMax;
+         i += gridDim.x * M3_BLOCK)
+    {
+        s.forced[i] = 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        s.plan->islands = 0;
+    }
+}
+
+// Adds up the islands' work: two a contact row, three a joint row, one a
+// mover.
+__global__ void __launch_bounds__(M3_BLOCK) m3IslandWorkKernel(const m3WorldView* views,
+                                                              const int32_t* order)
+{
+    const m3WorldView& w = views[order[0]];
+    const m3WorldScalars* sc = w.sc;
+    if (sc->status != 0)
+    {
+        return;
+    }
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    const int32_t gtid = blockIdx.x * M3_BLOCK + threadIdx.x;
+    const int32_t gstride = gridDim.x * M3_BLOCK;
+    for (int32_t i = gtid; i < s.plan->constraintCount; i += gstride)
+    {
+        const int2 p = s.conPair[i];
+        atomicAdd(&s.forced[IslandFind(s.parent, p.x >= 0 ? p.x : p.y)], 2);
+    }
+    for (int32_t r = gtid; r < s.plan->jointCount; r += gstride)
+    {
+        atomicAdd(&s.forced[IslandFind(s.parent, JointIslandBody(w, s.jointBodies[r]))], 3);
+    }
+    for (int32_t m = gtid; m < s.plan->moverCount; m += gstride)
+    {
+        const int32_t i = s.movers[m];
+        if (w.btype[i] != M3_BODY_DYNAMIC)
+        {
+            s.plan->islands = -1;
+        }
+        atomicAdd(&s.forced[IslandFind(s.parent, i)], 1);
+    }
+}
+
+// The islands' groups (per root, in s.forcedRoot), whether they are used,
+// and the tables cleared (one block).
+__global__ void __launch_bounds__(1024) m3IslandGroupKernel(const m3WorldView* views,
+                                                           const int32_t* order, int32_t groups)
+{
+    const m3WorldView& w = views[order[0]];
+    const m3WorldScalars* sc = w.sc;
+    if (sc->status != 0)
+    {
+        return;
+    }
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    const int32_t bodyMax = sc->bodyMax;
+    const int32_t tid = threadIdx.x;
+    const bool movedByHand = s.plan->islands < 0;
+    const m3IslandTables t = IslandTables(s, sc->pairCap, groups);
+    __shared__ int32_t s_most;
+    if (tid == 0)
+    {
+        s_most = 0;
+    }
+    __syncthreads();
+    for (int32_t i = tid; i < bodyMax; i += 1024)
+    {
+        s.forcedRoot[i] = s.forced[i];
+    }
+    __syncthreads();
+    const int32_t total = BlockExclusiveScan<1024>(s.forcedRoot, bodyMax);
+    // A group's work ends at most one island past its share.
+    const int64_t share = ((int64_t)total + groups - 1) / groups;
+    int32_t most = 0;
+    for (int32_t i = tid; i < bodyMax; i += 1024)
+    {
+        const int32_t work = s.forced[i];
+        const int64_t group = total > 0 ? (int64_t)s.forcedRoot[i] * groups / total : 0;
+        s.forcedRoot[i] = (int32_t)(group < groups ? group : groups - 1);
+        most = work > most ? work : most;
+    }
+    atomicMax(&s_most, most);
+    __syncthreads();
+    const int64_t levels = s.plan->levels > 0 ? s.plan->levels : 1;
+    const bool use = !movedByHand && t.fits && share + s_most <= M3_ISLAND_ROWS * levels;
+    __syncthreads();
+    if (tid == 0)
+    {
+        s.plan->islands = use ? 1 : 0;
+    }
+    if (!use)
+    {
+        return;
+    }
+    for (int32_t k = tid; k < t.contacts + t.joints + groups + 3; k += 1024)
+    {
+        t.contact[k] = 0;
+    }
+}
+
+// Rows and movers counted per (group, level), one entry on.
+__global__ void __launch_bounds__(M3_BLOCK) m3IslandCountKernel(const m3WorldView* views,
+                                                               const int32_t* order,
+                                                               int32_t groups)
+{
+    const m3WorldView& w = views[order[0]];
+    const m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    if (sc->status != 0 || s.plan->islands == 0)
+    {
+        return;
+    }
+    const m3IslandTables t = IslandTables(s, sc->pairCap, groups);
+    const int32_t levels = s.plan->levels;
+    const int32_t jointLevels = s.plan->jointLevels;
+    const int32_t gtid = blockIdx.x * M3_BLOCK + threadIdx.x;
+    const int32_t gstride = gridDim.x * M3_BLOCK;
+    for (int32_t i = gtid; i < s.plan->constraintCount; i += gstride)
+    {
+        const int2 p = s.conPair[i];
+        const int32_t group = s.forcedRoot[IslandFind(s.parent, p.x >= 0 ? p.x : p.y)];
+        atomicAdd(&t.contact[group * (levels + 1) + s.conLevel[i] + 1], 1);
+    }
+    for (int32_t r = gtid; r < s.plan->jointCount; r += gstride)
+    {
+        const int32_t group =
+            s.forcedRoot[IslandFind(s.parent, JointIslandBody(w, s.jointBodies[r]))];
+        atomicAdd(&t.joint[group * jointLevels + s.jointLevel[r] + 1], 1);
+    }
+    for (int32_t m = gtid; m < s.plan->moverCount; m += gstride)
+    {
+        atomicAdd(&t.mover[s.forcedRoot[IslandFind(s.parent, s.movers[m])] + 1], 1);
+    }
+}
+
+// The counts to starts, and the fill cursors (one block).
+__global__ void __launch_bounds__(1024) m3IslandStartKernel(const m3WorldView* views,
+                                                           const int32_t* order, int32_t groups)
+{
+    const m3WorldView& w = views[order[0]];
+    const m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    if (sc->status != 0 || s.plan->islands == 0)
+    {
+        return;
+    }
+    const m3IslandTables t = IslandTables(s, sc->pairCap, groups);
+    const int32_t tid = threadIdx.x;
+    // Entry k + 1 holds the count of k: an exclusive scan from entry 1
+    // leaves entry k + 1 the start of k, and the copy below moves it.
+    int32_t* tables[3] = {t.contact, t.joint, t.mover};
+    int32_t* fills[3] = {t.contactFill, t.jointFill, t.moverFill};
+    const int32_t sizes[3] = {t.contacts, t.joints, groups};
+    for (int32_t a = 0; a < 3; ++a)
+    {
+        const int32_t total = BlockExclusiveScan<1024>(tables[a] + 1, sizes[a]);
+        for (int32_t k = tid; k < sizes[a]; k += 1024)
+        {
+            fills[a][k] = tables[a][k + 1];
+        }
+        __syncthreads();
+        for (int32_t k = tid; k < sizes[a]; k += 1024)
+        {
+            tables[a][k] = fills[a][k];
+        }
+        if (tid == 0)
+        {
+            tables[a][sizes[a]] = total;
+        }
+        __syncthreads();
+    }
+}
+
+// Rows to their slots by (group, level), movers to their groups; the
+// overflow rows keep constraint order.
+__global__ void __launch_bounds__(M3_BLOCK) m3IslandFillKernel(const m3WorldView* views,
+                                                              const int32_t* order,
+                                                              int32_t groups)
+{
+    const m3WorldView& w = views[order[0]];
+    const m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    if (sc->status != 0 || s.plan->islands == 0)
+    {
+        return;
+    }
+    const m3IslandTables t = IslandTables(s, sc->pairCap, groups);
+    const int32_t levels = s.plan->levels;
+    const int32_t jointLevels = s.plan->jointLevels;
+    const int32_t constraintCount = s.plan->constraintCount;
+    const int32_t gtid = blockIdx.x * M3_BLOCK + threadIdx.x;
+    const int32_t gstride = gridDim.x * M3_BLOCK;
+    const auto groupOf = [&](int32_t i) {
+        const int2 p = s.conPair[i];
+        return s.forcedRoot[IslandFind(s.parent, p.x >= 0 ? p.x : p.y)];
+    };
+    for (int32_t i = gtid; i < constraintCount; i += gstride)
+    {
+        const int32_t level = s.conLevel[i];
+        if (level < levels)
+        {
+            const int32_t slot =
+                atomicAdd(&t.contactFill[groupOf(i) * (levels + 1) + level], 1);
+            s.lists[slot] = i;
+            s.conSlot[i] = slot;
+        }
+    }
+    if (gtid == 0 && s.levelStart[levels + 1] > s.levelStart[levels])
+    {
+        for (int32_t i = 0; i < constraintCount; ++i)
+        {
+            if (s.conLevel[i] == levels)
+            {
+                const int32_t slot = t.contactFill[groupOf(i) * (levels + 1) + levels]++;
+                s.lists[slot] = i;
+                s.conSlot[i] = slot;
+            }
+        }
+    }
+    for (int32_t r = gtid; r < s.plan->jointCount; r += gstride)
+    {
+        const int32_t group =
+            s.forcedRoot[IslandFind(s.parent, JointIslandBody(w, s.jointBodies[r]))];
+        s.jointOrder[atomicAdd(&t.jointFill[group * jointLevels + s.jointLevel[r]], 1)] = r;
+    }
+    // The groups' movers (the colouring's claims are spent).
+    for (int32_t m = gtid; m < s.plan->moverCount; m += gstride)
+    {
+        const int32_t i = s.movers[m];
+        s.colorMin[atomicAdd(&t.moverFill[s.forcedRoot[IslandFind(s.parent, i)]], 1)] = i;
+    }
+}
+
+// The substep loop (solver.c:4085-4203), a group a block.
+__global__ void __launch_bounds__(M3_ISLAND_THREADS)
+    m3IslandSubstepKernel(const m3WorldView* views, const int32_t* order, float dt,
+                          int32_t substeps)
+{
+    const m3WorldView& w = views[order[0]];
+    m3WorldScalars* sc = w.sc;
+    m3Scratch s;
+    ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap);
+    if (sc->status != 0 || s.plan->islands == 0)
+    {
+        return;
+    }
+    const m3IslandTables t = IslandTables(s, sc->pairCap, (int32_t)gridDim.x);
+    const int32_t tid = threadIdx.x;
+    const int32_t levels = s.plan->levels;
+    const int32_t jointLevels = s.plan->jointLevels;
+    const int32_t* contactStart = t.contact + (int32_t)blockIdx.x * (levels + 1);
+    const int32_t* jointStart = t.joint + (int32_t)blockIdx.x * jointLevels;
+    const int32_t m0 = t.mover[blockIdx.x];
+    const int32_t m1 = t.mover[blockIdx.x + 1];
+    const int32_t* movers = s.colorMin;
+    const m3real h = dt / (m3real)substeps;
+    const m3real invH = h > 0.0f ? 1.0f / h : 0.0f;
+    const m3real pushMax = sc->contactPushMaxSpeed;
+    m3Vec3* dP = s.deltaPos;
+    m3Quat* dQ = s.deltaRot;
+    const m3Mat3* invI = s.bodyInvI;
+    const bool lead = blockIdx.x == 0 && tid == 0;
+    long long t_phase = clock64();
+#define M3_ISLAND_MARK(k)                                                                          \
+    if (lead)                                                                                      \
+    {                                                                                              \
+        long long now_ = clock64();                                                                \
+        sc->phase[k] += (uint64_t)(now_ - t_phase);                                                \
+        t_phase = now_;                                                                            \
+    }
+    const auto contact = [&](int32_t slot, int32_t which) {
+        const m3ConRef c = m3ConAt(s.rows, slot);
+        if (which == 0)
+        {
+            m3WarmStartContact(w, c, invI);
+        }
+        else
+        {
+            m3SolveContact(w, c, invI, dP, dQ, invH, pushMax, which == 1);
+        }
+    };
+    const auto pass = [&](int32_t which) {
+        for (int32_t level = 0; level < levels; ++level)
+        {
+            int32_t j0 = 0;
+            int32_t nj = 0;
+            if (level < jointLevels)
+            {
+                j0 = jointStart[level];
+                nj = jointStart[level + 1] - j0;
+            }
+            const int32_t c0 = contactStart[level];
+            const int32_t nc = contactStart[level + 1] - c0;
+            if (nj + nc == 0)
+            {
+                continue;
+            }
+            for (int32_t r = tid; r < nj + nc; r += M3_ISLAND_THREADS)
+            {
+                if (r < nj)
+                {
+                    m3JointDev* row = &s.joints[s.jointOrder[j0 + r]];
+                    if (which == 0)
+                    {
+                        m3WarmStartJoint(w, row, dQ);
+                    }
+                    else
+                    {
+                        m3SolveJoint(w, row, dP, dQ, h, invH, which == 1);
+                    }
+                }
+                else
+                {
+                    contact(c0 + (r - nj), which);
+                }
+            }
+            __syncthreads();
+        }
+        const int32_t o0 = contactStart[levels];
+        const int32_t o1 = contactStart[levels + 1];
+        if (o1 > o0)
+        {
+            if (tid == 0)
+            {
+                for (int32_t k = o0; k < o1; ++k)
+                {
+                    contact(k, which);
+                }
+            }
+            __syncthreads();
+        }
+    };
+    for (int32_t sub = 0; sub < substeps; ++sub)
+    {
+        for (int32_t m = m0 + tid; m < m1; m += M3_ISLAND_THREADS)
+        {
+            m3IntegrateVelocity(w, movers[m], h);
+        }
+        __syncthreads();
+        M3_ISLAND_MARK(M3_PHASE_INTEGRATE_V)
+        pass(0);
+        M3_ISLAND_MARK(M3_PHASE_WARM)
+        pass(1);
+        M3_ISLAND_MARK(M3_PHASE_SOLVE)
+        for (int32_t m = m0 + tid; m < m1; m += M3_ISLAND_THREADS)
+        {
+            m3IntegratePosition(w, movers[m], h, dP, dQ);
+        }
+        __syncthreads();
+        M3_ISLAND_MARK(M3_PHASE_INTEGRATE_P)
+        pass(2);
+        M3_ISLAND_MARK(M3_PHASE_RELAX)
+    }
+#undef M3_ISLAND_MARK
 }
 
 // A wide world's contact rows (solver.c:261-405), one per thread over
@@ -5670,7 +6097,17 @@ static int32_t BroadSortCap(int32_t shapes)
 static void LaunchWideSubstep(const m3WorldView* views, const int32_t* order, float dt,
                               int32_t substeps, int32_t blocks)
 {
+    const int32_t wide = 2 * s_smCount;
+    const int32_t groups = s_smCount;
+    m3IslandClearKernel<<<wide, M3_BLOCK>>>(views, order);
+    m3IslandWorkKernel<<<wide, M3_BLOCK>>>(views, order);
+    m3IslandGroupKernel<<<1, 1024>>>(views, order, groups);
+    m3IslandCountKernel<<<wide, M3_BLOCK>>>(views, order, groups);
+    m3IslandStartKernel<<<1, 1024>>>(views, order, groups);
+    m3IslandFillKernel<<<wide, M3_BLOCK>>>(views, order, groups);
     m3WideRowsKernel<<<4 * s_smCount, 256>>>(views, order, dt, substeps);
+    m3IslandSubstepKernel<<<groups, M3_ISLAND_THREADS>>>(views, order, dt, substeps);
+    s_launches += 7;
     void* args[] = {(void*)&views, (void*)&order, (void*)&dt, (void*)&substeps};
     cudaLaunchCooperativeKernel((const void*)m3WideSubstepKernel<256>, dim3(blocks), dim3(256),
                                 args, 0, 0);
