@@ -188,29 +188,35 @@ __device__ void m3PrepareJoint(const m3WorldView& w, m3JointDev* c, int32_t j, m
 // One joint's warm start (solver.c:1044-1209 loop body).
 __device__ void m3WarmStartJoint(const m3WorldView& w, m3JointDev* c, const m3Quat* deltaRot)
 {
+    const int32_t a = c->bodyA;
+    const int32_t b = c->bodyB;
+    const m3Vec3 vA = w.v[a];
+    const m3Vec3 wA = w.w[a];
+    const m3Vec3 vB = w.v[b];
+    const m3Vec3 wB = w.w[b];
+    const m3real mA = c->invMassA;
+    const m3real mB = c->invMassB;
+    const m3Mat3 iA = c->invIA;
+    const m3Mat3 iB = c->invIB;
+    const m3Vec3 rA = m3RotateVec3(deltaRot[a], c->rA);
+    const m3Vec3 rB = m3RotateVec3(deltaRot[b], c->rB);
+    m3Vec3 angularImpulse = v3(0.0f, 0.0f, 0.0f);
+    if (c->type == 1)
     {
-        m3Vec3 rA = m3RotateVec3(deltaRot[c->bodyA], c->rA);
-        m3Vec3 rB = m3RotateVec3(deltaRot[c->bodyB], c->rB);
-        m3Vec3 angularImpulse = v3(0.0f, 0.0f, 0.0f);
-        if (c->type == 1)
-        {
-            m3real axial = c->springImpulseV.x + c->motorImpulse + c->lowerImpulse - c->upperImpulse;
-            angularImpulse = m3Add3(m3MulSV3(c->perpImpulseX, c->perpAxisX),
-                                    m3MulSV3(c->perpImpulseY, c->perpAxisY));
-            angularImpulse = m3Add3(angularImpulse, m3MulSV3(axial, c->rotationAxis));
-        }
-        else if (c->type == 3)
-        {
-            angularImpulse = c->angularImpulse;
-        }
-        m3Vec3 totalLinear = m3Add3(c->impulse, v3(0.0f, 0.0f, 0.0f));
-        w.v[c->bodyA] = m3Sub3(w.v[c->bodyA], m3MulSV3(c->invMassA, totalLinear));
-        w.w[c->bodyA] = m3Sub3(w.w[c->bodyA],
-                               m3MulMV3(c->invIA, m3Add3(m3Cross3(rA, totalLinear), angularImpulse)));
-        w.v[c->bodyB] = m3Add3(w.v[c->bodyB], m3MulSV3(c->invMassB, totalLinear));
-        w.w[c->bodyB] = m3Add3(w.w[c->bodyB],
-                               m3MulMV3(c->invIB, m3Add3(m3Cross3(rB, totalLinear), angularImpulse)));
+        m3real axial = c->springImpulseV.x + c->motorImpulse + c->lowerImpulse - c->upperImpulse;
+        angularImpulse = m3Add3(m3MulSV3(c->perpImpulseX, c->perpAxisX),
+                                m3MulSV3(c->perpImpulseY, c->perpAxisY));
+        angularImpulse = m3Add3(angularImpulse, m3MulSV3(axial, c->rotationAxis));
     }
+    else if (c->type == 3)
+    {
+        angularImpulse = c->angularImpulse;
+    }
+    const m3Vec3 totalLinear = m3Add3(c->impulse, v3(0.0f, 0.0f, 0.0f));
+    w.v[a] = m3Sub3(vA, m3MulSV3(mA, totalLinear));
+    w.w[a] = m3Sub3(wA, m3MulMV3(iA, m3Add3(m3Cross3(rA, totalLinear), angularImpulse)));
+    w.v[b] = m3Add3(vB, m3MulSV3(mB, totalLinear));
+    w.w[b] = m3Add3(wB, m3MulMV3(iB, m3Add3(m3Cross3(rB, totalLinear), angularImpulse)));
 }
 
 // One-sided angular limit row (solver.c:1374-1430 form).
@@ -243,16 +249,24 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
                              const m3Quat* deltaRot, m3real hSub, m3real invHSub, bool useBias)
 {
     {
-        m3Vec3 rA = m3RotateVec3(deltaRot[c->bodyA], c->rA);
-        m3Vec3 rB = m3RotateVec3(deltaRot[c->bodyB], c->rB);
-        m3Vec3 vA = w.v[c->bodyA];
-        m3Vec3 wA = w.w[c->bodyA];
-        m3Vec3 vB = w.v[c->bodyB];
-        m3Vec3 wB = w.w[c->bodyB];
+        const int32_t bodyA = c->bodyA;
+        const int32_t bodyB = c->bodyB;
+        const m3Mat3 iA = c->invIA;
+        const m3Mat3 iB = c->invIB;
+        const m3real mA = c->invMassA;
+        const m3real mB = c->invMassB;
+        const m3Quat dqA = deltaRot[bodyA];
+        const m3Quat dqB = deltaRot[bodyB];
+        m3Vec3 rA = m3RotateVec3(dqA, c->rA);
+        m3Vec3 rB = m3RotateVec3(dqB, c->rB);
+        const m3Vec3 vA = w.v[bodyA];
+        m3Vec3 wA = w.w[bodyA];
+        const m3Vec3 vB = w.v[bodyB];
+        m3Vec3 wB = w.w[bodyB];
         if (c->type == 1)
         {
-            m3Quat quatA = m3MulQuat(deltaRot[c->bodyA], c->frameQA);
-            m3Quat quatB = m3MulQuat(deltaRot[c->bodyB], c->frameQB);
+            m3Quat quatA = m3MulQuat(dqA, c->frameQA);
+            m3Quat quatB = m3MulQuat(dqB, c->frameQB);
             if (quatA.x * quatB.x + quatA.y * quatB.y + quatA.z * quatB.z + quatA.w * quatB.w <
                 0.0f)
             {
@@ -269,8 +283,8 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
                 newImpulse = m3MaxF(-maxImpulse, m3MinF(maxImpulse, newImpulse));
                 delta = newImpulse - c->motorImpulse;
                 c->motorImpulse = newImpulse;
-                wA = m3Sub3(wA, m3MulSV3(delta, m3MulMV3(c->invIA, axis)));
-                wB = m3Add3(wB, m3MulSV3(delta, m3MulMV3(c->invIB, axis)));
+                wA = m3Sub3(wA, m3MulSV3(delta, m3MulMV3(iA, axis)));
+                wB = m3Add3(wB, m3MulSV3(delta, m3MulMV3(iB, axis)));
             }
             if ((c->flags & 1) != 0)
             {
@@ -279,15 +293,15 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
                     m3real cdot = m3Dot3(m3Sub3(wB, wA), axis);
                     m3real delta = m3LimitRow(angle - c->lowerLimit, cdot, c->axialMass,
                                               &c->lowerImpulse, c->softness, invHSub, useBias);
-                    wA = m3Sub3(wA, m3MulSV3(delta, m3MulMV3(c->invIA, axis)));
-                    wB = m3Add3(wB, m3MulSV3(delta, m3MulMV3(c->invIB, axis)));
+                    wA = m3Sub3(wA, m3MulSV3(delta, m3MulMV3(iA, axis)));
+                    wB = m3Add3(wB, m3MulSV3(delta, m3MulMV3(iB, axis)));
                 }
                 {
                     m3real cdot = m3Dot3(m3Sub3(wA, wB), axis);
                     m3real delta = m3LimitRow(c->upperLimit - angle, cdot, c->axialMass,
                                               &c->upperImpulse, c->softness, invHSub, useBias);
-                    wA = m3Add3(wA, m3MulSV3(delta, m3MulMV3(c->invIA, axis)));
-                    wB = m3Sub3(wB, m3MulSV3(delta, m3MulMV3(c->invIB, axis)));
+                    wA = m3Add3(wA, m3MulSV3(delta, m3MulMV3(iA, axis)));
+                    wB = m3Sub3(wB, m3MulSV3(delta, m3MulMV3(iB, axis)));
                 }
             }
             {
@@ -306,8 +320,8 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
                     massScale = c->softness.massScale;
                     impulseScale = c->softness.impulseScale;
                 }
-                m3Vec3 sumX = m3Add3(m3MulMV3(c->invIA, perpX), m3MulMV3(c->invIB, perpX));
-                m3Vec3 sumY = m3Add3(m3MulMV3(c->invIA, perpY), m3MulMV3(c->invIB, perpY));
+                m3Vec3 sumX = m3Add3(m3MulMV3(iA, perpX), m3MulMV3(iB, perpX));
+                m3Vec3 sumY = m3Add3(m3MulMV3(iA, perpY), m3MulMV3(iB, perpY));
                 m3real kxx = m3Dot3(perpX, sumX);
                 m3real kyy = m3Dot3(perpY, sumY);
                 m3real kxy = m3Dot3(perpX, sumY);
@@ -328,15 +342,9 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
                 c->perpImpulseX += deltaX;
                 c->perpImpulseY += deltaY;
                 m3Vec3 angular = m3Add3(m3MulSV3(deltaX, perpX), m3MulSV3(deltaY, perpY));
-                wA = m3Sub3(wA, m3MulMV3(c->invIA, angular));
-                wB = m3Add3(wB, m3MulMV3(c->invIB, angular));
+                wA = m3Sub3(wA, m3MulMV3(iA, angular));
+                wB = m3Add3(wB, m3MulMV3(iB, angular));
             }
-            w.w[c->bodyA] = wA;
-            w.w[c->bodyB] = wB;
-            vA = w.v[c->bodyA];
-            wA = w.w[c->bodyA];
-            vB = w.v[c->bodyB];
-            wB = w.w[c->bodyB];
         }
         else if (c->type == 3)
         {
@@ -345,8 +353,8 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
             m3real impulseScale = 0.0f;
             if (useBias)
             {
-                m3Quat quatA = m3MulQuat(deltaRot[c->bodyA], c->frameQA);
-                m3Quat quatB = m3MulQuat(deltaRot[c->bodyB], c->frameQB);
+                m3Quat quatA = m3MulQuat(dqA, c->frameQA);
+                m3Quat quatB = m3MulQuat(dqB, c->frameQB);
                 m3Quat relQ = m3MulQuat(m3Conj(quatA), quatB);
                 m3Vec3 rotVec = m3QuatToRotationVec(relQ);
                 m3Vec3 cErr = m3RotateVec3(quatA, rotVec);
@@ -355,18 +363,15 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
                 impulseScale = c->softness.impulseScale;
             }
             m3Mat3 k;
-            k.cx = m3Add3(m3MulMV3(c->invIA, v3(1.0f, 0.0f, 0.0f)),
-                          m3MulMV3(c->invIB, v3(1.0f, 0.0f, 0.0f)));
-            k.cy = m3Add3(m3MulMV3(c->invIA, v3(0.0f, 1.0f, 0.0f)),
-                          m3MulMV3(c->invIB, v3(0.0f, 1.0f, 0.0f)));
-            k.cz = m3Add3(m3MulMV3(c->invIA, v3(0.0f, 0.0f, 1.0f)),
-                          m3MulMV3(c->invIB, v3(0.0f, 0.0f, 1.0f)));
+            k.cx = m3Add3(m3MulMV3(iA, v3(1.0f, 0.0f, 0.0f)), m3MulMV3(iB, v3(1.0f, 0.0f, 0.0f)));
+            k.cy = m3Add3(m3MulMV3(iA, v3(0.0f, 1.0f, 0.0f)), m3MulMV3(iB, v3(0.0f, 1.0f, 0.0f)));
+            k.cz = m3Add3(m3MulMV3(iA, v3(0.0f, 0.0f, 1.0f)), m3MulMV3(iB, v3(0.0f, 0.0f, 1.0f)));
             m3Vec3 cdotRot = m3Sub3(wB, wA);
             m3Vec3 sol = m3Solve3(&k, m3Add3(cdotRot, bias));
             m3Vec3 delta = m3Sub3(m3MulSV3(-massScale, sol), m3MulSV3(impulseScale, c->angularImpulse));
             c->angularImpulse = m3Add3(c->angularImpulse, delta);
-            wA = m3Sub3(wA, m3MulMV3(c->invIA, delta));
-            wB = m3Add3(wB, m3MulMV3(c->invIB, delta));
+            wA = m3Sub3(wA, m3MulMV3(iA, delta));
+            wB = m3Add3(wB, m3MulMV3(iB, delta));
         }
 
         // The shared point constraint (solver.c:2656-2701).
@@ -377,7 +382,7 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
         if (useBias)
         {
             m3Vec3 separation =
-                m3Add3(m3Add3(m3Sub3(deltaPos[c->bodyB], deltaPos[c->bodyA]), m3Sub3(rB, rA)),
+                m3Add3(m3Add3(m3Sub3(deltaPos[bodyB], deltaPos[bodyA]), m3Sub3(rB, rA)),
                        c->deltaCenter);
             bias = m3MulSV3(c->softness.biasRate, separation);
             massScale = c->softness.massScale;
@@ -388,17 +393,17 @@ __device__ void m3SolveJoint(const m3WorldView& w, m3JointDev* c, const m3Vec3* 
         for (int32_t a = 0; a < 3; ++a)
         {
             m3Vec3 e = v3(a == 0 ? 1.0f : 0.0f, a == 1 ? 1.0f : 0.0f, a == 2 ? 1.0f : 0.0f);
-            m3Vec3 tA = m3Cross3(rA, m3MulMV3(c->invIA, m3Cross3(rA, e)));
-            m3Vec3 tB = m3Cross3(rB, m3MulMV3(c->invIB, m3Cross3(rB, e)));
-            *cols[a] = m3Sub3(m3MulSV3(c->invMassA + c->invMassB, e), m3Add3(tA, tB));
+            m3Vec3 tA = m3Cross3(rA, m3MulMV3(iA, m3Cross3(rA, e)));
+            m3Vec3 tB = m3Cross3(rB, m3MulMV3(iB, m3Cross3(rB, e)));
+            *cols[a] = m3Sub3(m3MulSV3(mA + mB, e), m3Add3(tA, tB));
         }
         m3Vec3 b = m3Solve3(&k, m3Add3(cdot, bias));
         m3Vec3 impulse = m3Sub3(m3MulSV3(-massScale, b), m3MulSV3(impulseScale, c->impulse));
         c->impulse = m3Add3(c->impulse, impulse);
-        w.v[c->bodyA] = m3Sub3(vA, m3MulSV3(c->invMassA, impulse));
-        w.w[c->bodyA] = m3Sub3(wA, m3MulMV3(c->invIA, m3Cross3(rA, impulse)));
-        w.v[c->bodyB] = m3Add3(vB, m3MulSV3(c->invMassB, impulse));
-        w.w[c->bodyB] = m3Add3(wB, m3MulMV3(c->invIB, m3Cross3(rB, impulse)));
+        w.v[bodyA] = m3Sub3(vA, m3MulSV3(mA, impulse));
+        w.w[bodyA] = m3Sub3(wA, m3MulMV3(iA, m3Cross3(rA, impulse)));
+        w.v[bodyB] = m3Add3(vB, m3MulSV3(mB, impulse));
+        w.w[bodyB] = m3Add3(wB, m3MulMV3(iB, m3Cross3(rB, impulse)));
     }
 }
 

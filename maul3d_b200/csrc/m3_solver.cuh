@@ -241,19 +241,79 @@ __device__ __forceinline__ m3ConBodies m3LoadConBodies(const m3ConRef& c, const 
     return cb;
 }
 
+// The velocities of a row's two bodies, held in registers from the row's
+// first read to its last write (the two bodies of a row differ, and no
+// other row of its level touches them).  Through memory every point's
+// impulse was a store and a load of both bodies that the next point waited
+// for.  Only a dynamic body's velocities are written.
+struct m3ConVelocities
+{
+    m3Vec3 vA;
+    m3Vec3 wA;
+    m3Vec3 vB;
+    m3Vec3 wB;
+};
+
+__device__ __forceinline__ m3ConVelocities m3LoadConVelocities(const m3WorldView& w,
+                                                               const m3ConBodies& cb)
+{
+    m3ConVelocities u;
+    u.vA = w.v[cb.a];
+    u.wA = w.w[cb.a];
+    u.vB = w.v[cb.b];
+    u.wB = w.w[cb.b];
+    return u;
+}
+
+__device__ __forceinline__ void m3StoreConVelocities(const m3WorldView& w, const m3ConBodies& cb,
+                                                     const m3ConVelocities& u)
+{
+    if (cb.dynA)
+    {
+        w.v[cb.a] = u.vA;
+        w.w[cb.a] = u.wA;
+    }
+    if (cb.dynB)
+    {
+        w.v[cb.b] = u.vB;
+        w.w[cb.b] = u.wB;
+    }
+}
+
+// The relative velocity of the bodies' points at arms rA and rB.
+__device__ __forceinline__ m3Vec3 m3RelativeVelocity(const m3ConVelocities& u, m3Vec3 rA,
+                                                     m3Vec3 rB)
+{
+    return m3Sub3(m3Add3(u.vB, m3Cross3(u.wB, rB)), m3Add3(u.vA, m3Cross3(u.wA, rA)));
+}
+
 // solver.c:105-121
-__device__ __forceinline__ void m3ApplyImpulseRow(const m3WorldView& w, const m3ConBodies& cb,
+__device__ __forceinline__ void m3ApplyImpulseRow(m3ConVelocities& u, const m3ConBodies& cb,
                                                   m3Vec3 impulse, m3Vec3 rsA, m3Vec3 rsB)
 {
     if (cb.dynA)
     {
-        w.v[cb.a] = m3Sub3(w.v[cb.a], m3MulSV3(cb.mA, impulse));
-        w.w[cb.a] = m3Sub3(w.w[cb.a], m3MulMV3(cb.iA, m3Cross3(rsA, impulse)));
+        u.vA = m3Sub3(u.vA, m3MulSV3(cb.mA, impulse));
+        u.wA = m3Sub3(u.wA, m3MulMV3(cb.iA, m3Cross3(rsA, impulse)));
     }
     if (cb.dynB)
     {
-        w.v[cb.b] = m3Add3(w.v[cb.b], m3MulSV3(cb.mB, impulse));
-        w.w[cb.b] = m3Add3(w.w[cb.b], m3MulMV3(cb.iB, m3Cross3(rsB, impulse)));
+        u.vB = m3Add3(u.vB, m3MulSV3(cb.mB, impulse));
+        u.wB = m3Add3(u.wB, m3MulMV3(cb.iB, m3Cross3(rsB, impulse)));
+    }
+}
+
+// An angular impulse on both bodies.
+__device__ __forceinline__ void m3ApplyTwistRow(m3ConVelocities& u, const m3ConBodies& cb,
+                                                m3Vec3 tw)
+{
+    if (cb.dynA)
+    {
+        u.wA = m3Sub3(u.wA, m3MulMV3(cb.iA, tw));
+    }
+    if (cb.dynB)
+    {
+        u.wB = m3Add3(u.wB, m3MulMV3(cb.iB, tw));
     }
 }
 
@@ -461,6 +521,7 @@ __device__ void m3WarmStartContact(const m3WorldView& w, const m3ConRef& c, cons
     const m3real f1 = c.a(M3A_FRICTION1);
     const m3real f2 = c.a(M3A_FRICTION2);
     const m3real twist = c.a(M3A_TWIST);
+    m3ConVelocities u = m3LoadConVelocities(w, cb);
     const m3Vec3 rolling = v3(c.a(M3A_ROLLING), c.a(M3A_ROLLING + 1), c.a(M3A_ROLLING + 2));
 #pragma unroll
     for (int32_t k = 0; k < M3_MANIFOLD_MAX_POINTS; ++k)
@@ -468,20 +529,13 @@ __device__ void m3WarmStartContact(const m3WorldView& w, const m3ConRef& c, cons
         if (k < pc)
         {
             const int32_t p = M3C_POINT0 + M3C_POINT_WORDS * k;
-            m3ApplyImpulseRow(w, cb, m3MulSV3(imp[k], normal), c.v(p), c.v(p + 3));
+            m3ApplyImpulseRow(u, cb, m3MulSV3(imp[k], normal), c.v(p), c.v(p + 3));
         }
     }
     m3Vec3 f = m3Add3(m3MulSV3(f1, c.v(M3C_T1)), m3MulSV3(f2, c.v(M3C_T2)));
-    m3ApplyImpulseRow(w, cb, f, c.v(M3C_ORIGIN_A), c.v(M3C_ORIGIN_B));
-    m3Vec3 tw = m3Add3(m3MulSV3(twist, normal), rolling);
-    if (cb.dynA)
-    {
-        w.w[cb.a] = m3Sub3(w.w[cb.a], m3MulMV3(cb.iA, tw));
-    }
-    if (cb.dynB)
-    {
-        w.w[cb.b] = m3Add3(w.w[cb.b], m3MulMV3(cb.iB, tw));
-    }
+    m3ApplyImpulseRow(u, cb, f, c.v(M3C_ORIGIN_A), c.v(M3C_ORIGIN_B));
+    m3ApplyTwistRow(u, cb, m3Add3(m3MulSV3(twist, normal), rolling));
+    m3StoreConVelocities(w, cb, u);
 }
 
 // solver.c:430-574
@@ -500,6 +554,7 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
         imp[k] = k < pc ? c.a(M3A_NORMAL + k) : 0.0f;
         tot[k] = k < pc ? c.a(M3A_TOTAL_NORMAL + k) : 0.0f;
     }
+    m3ConVelocities u = m3LoadConVelocities(w, cb);
     m3real passNormal = 0.0f;
     m3real twistLimit = 0.0f;
     const m3Quat qA = deltaRot[cb.a];
@@ -531,7 +586,7 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
                 massScale = c.f(M3C_SOFT + 1);
                 impulseScale = c.f(M3C_SOFT + 2);
             }
-            m3real vn = m3Dot3(m3Sub3(m3VelocityAt(w, cb.b, rB), m3VelocityAt(w, cb.a, rA)), normal);
+            m3real vn = m3Dot3(m3RelativeVelocity(u, rA, rB), normal);
             m3real impulse = -c.f(p + 7) * massScale * (vn + bias) - impulseScale * imp[k];
             m3real newImpulse = m3MaxF(imp[k] + impulse, 0.0f);
             impulse = newImpulse - imp[k];
@@ -539,7 +594,7 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
             tot[k] += newImpulse;
             passNormal += newImpulse;
             twistLimit += c.f(p + 8) * newImpulse;
-            m3ApplyImpulseRow(w, cb, m3MulSV3(impulse, normal), rA, rB);
+            m3ApplyImpulseRow(u, cb, m3MulSV3(impulse, normal), rA, rB);
         }
     }
 #pragma unroll
@@ -553,11 +608,12 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
     }
     if (useBias)
     {
+        m3StoreConVelocities(w, cb, u);
         return;
     }
     const m3real friction = c.f(M3C_FRICTION);
     {
-        m3Vec3 wRel = m3Sub3(w.w[cb.b], w.w[cb.a]);
+        m3Vec3 wRel = m3Sub3(u.wB, u.wA);
         m3real twistSpeed = m3Dot3(normal, wRel);
         m3real maxTwist = friction * twistLimit;
         m3real delta = -c.f(M3C_TWIST_MASS) * twistSpeed;
@@ -573,15 +629,7 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
         }
         delta = newTwist - oldTwist;
         c.a(M3A_TWIST) = newTwist;
-        m3Vec3 tw = m3MulSV3(delta, normal);
-        if (cb.dynA)
-        {
-            w.w[cb.a] = m3Sub3(w.w[cb.a], m3MulMV3(cb.iA, tw));
-        }
-        if (cb.dynB)
-        {
-            w.w[cb.b] = m3Add3(w.w[cb.b], m3MulMV3(cb.iB, tw));
-        }
+        m3ApplyTwistRow(u, cb, m3MulSV3(delta, normal));
     }
     const m3real rollingResistance = c.f(M3C_ROLLING);
     if (rollingResistance > 0.0f)
@@ -592,7 +640,7 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
         const m3Mat3 rollingK = c.m(M3C_ROLLING_K);
         const m3Vec3 rollingImpulse =
             v3(c.a(M3A_ROLLING), c.a(M3A_ROLLING + 1), c.a(M3A_ROLLING + 2));
-        m3Vec3 wRel = m3Sub3(w.w[cb.b], w.w[cb.a]);
+        m3Vec3 wRel = m3Sub3(u.wB, u.wA);
         m3Vec3 delta = m3MulSV3(-1.0f, m3Solve3(&rollingK, wRel));
         m3Vec3 accum = m3Add3(rollingImpulse, delta);
         m3real maxRoll = rollingResistance * passNormal;
@@ -605,8 +653,16 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
         c.a(M3A_ROLLING) = accum.x;
         c.a(M3A_ROLLING + 1) = accum.y;
         c.a(M3A_ROLLING + 2) = accum.z;
-        w.w[cb.a] = m3Sub3(w.w[cb.a], m3MulMV3(cb.iA, delta));
-        w.w[cb.b] = m3Add3(w.w[cb.b], m3MulMV3(cb.iB, delta));
+        u.wA = m3Sub3(u.wA, m3MulMV3(cb.iA, delta));
+        u.wB = m3Add3(u.wB, m3MulMV3(cb.iB, delta));
+        if (!cb.dynA)
+        {
+            w.w[cb.a] = u.wA;
+        }
+        if (!cb.dynB)
+        {
+            w.w[cb.b] = u.wB;
+        }
     }
     {
         const m3Vec3 t1 = c.v(M3C_T1);
@@ -618,7 +674,7 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
         const m3real k22 = c.f(M3C_K22);
         const m3real oldF1 = c.a(M3A_FRICTION1);
         const m3real oldF2 = c.a(M3A_FRICTION2);
-        m3Vec3 vrel = m3Sub3(m3VelocityAt(w, cb.b, originB), m3VelocityAt(w, cb.a, originA));
+        m3Vec3 vrel = m3RelativeVelocity(u, originA, originB);
         m3real vt1 = m3Dot3(vrel, t1) - c.f(M3C_TANGENT_V1);
         m3real vt2 = m3Dot3(vrel, t2) - c.f(M3C_TANGENT_V2);
         m3real f1 = oldF1 - (k11 * vt1 + k12 * vt2);
@@ -636,8 +692,9 @@ __device__ void m3SolveContact(const m3WorldView& w, const m3ConRef& c, const m3
         m3real d2 = f2 - oldF2;
         c.a(M3A_FRICTION1) = f1;
         c.a(M3A_FRICTION2) = f2;
-        m3ApplyImpulseRow(w, cb, m3Add3(m3MulSV3(d1, t1), m3MulSV3(d2, t2)), originA, originB);
+        m3ApplyImpulseRow(u, cb, m3Add3(m3MulSV3(d1, t1), m3MulSV3(d2, t2)), originA, originB);
     }
+    m3StoreConVelocities(w, cb, u);
 }
 
 // solver.c:2879-2906 (one constraint's points, in order).
@@ -652,6 +709,7 @@ __device__ void m3RestituteContact(const m3WorldView& w, const m3ConRef& c, cons
     const m3ConBodies cb = m3LoadConBodies(c, invI);
     const int32_t pc = c.n(M3C_POINTS);
     const m3Vec3 normal = c.v(M3C_NORMAL);
+    m3ConVelocities u = m3LoadConVelocities(w, cb);
     for (int32_t k = 0; k < pc; ++k)
     {
         const int32_t p = M3C_POINT0 + M3C_POINT_WORDS * k;
@@ -662,14 +720,15 @@ __device__ void m3RestituteContact(const m3WorldView& w, const m3ConRef& c, cons
         }
         const m3Vec3 rA = c.v(p);
         const m3Vec3 rB = c.v(p + 3);
-        m3real vn = m3Dot3(m3Sub3(m3VelocityAt(w, cb.b, rB), m3VelocityAt(w, cb.a, rA)), normal);
+        m3real vn = m3Dot3(m3RelativeVelocity(u, rA, rB), normal);
         m3real impulse = -c.f(p + 7) * (vn + restitution * relativeVelocity);
         const m3real old = c.a(M3A_NORMAL + k);
         m3real newImpulse = m3MaxF(old + impulse, 0.0f);
         impulse = newImpulse - old;
         c.a(M3A_NORMAL + k) = newImpulse;
-        m3ApplyImpulseRow(w, cb, m3MulSV3(impulse, normal), rA, rB);
+        m3ApplyImpulseRow(u, cb, m3MulSV3(impulse, normal), rA, rB);
     }
+    m3StoreConVelocities(w, cb, u);
 }
 
 // solver.c:2979-3039 without the hit-event stream (observer only).

@@ -3024,8 +3024,9 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3PrepareKernel(const m3WorldV
 // ---------------------------------------------------------------------
 // Kernel 3: the substep loop, restitution and the impulse store
 // ---------------------------------------------------------------------
-// NT threads per world (one of the size classes below); MIN_BLOCKS keeps
-// the register budget at 128 per thread for every class.
+// NT threads per world (one of the size classes below); MIN_BLOCKS sets
+// the register budget: 128 per thread for the classes, up to 255 where a
+// world has its SM to itself.
 template <int NT, int MIN_BLOCKS>
 __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3SubstepKernel(const m3WorldView* views,
                                                             const int32_t* order, int32_t count,
@@ -4796,9 +4797,14 @@ __global__ void __launch_bounds__(M3_ISLAND_THREADS)
             {
                 continue;
             }
-            for (int32_t r = tid; r < nj + nc; r += M3_ISLAND_THREADS)
+            // Joint rows on the first warps, contact rows on the others:
+            // the two kinds never diverge inside a warp.
+            const int32_t jointWarps =
+                min((nj + 31) / 32, M3_ISLAND_THREADS / 32 - (nc > 0 ? 1 : 0));
+            const int32_t jointThreads = 32 * jointWarps;
+            if (tid < jointThreads)
             {
-                if (r < nj)
+                for (int32_t r = tid; r < nj; r += jointThreads)
                 {
                     m3JointDev* row = &s.joints[s.jointOrder[j0 + r]];
                     if (which == 0)
@@ -4810,9 +4816,13 @@ __global__ void __launch_bounds__(M3_ISLAND_THREADS)
                         m3SolveJoint(w, row, dP, dQ, h, invH, which == 1);
                     }
                 }
-                else
+            }
+            else
+            {
+                for (int32_t r = tid - jointThreads; r < nc;
+                     r += M3_ISLAND_THREADS - jointThreads)
                 {
-                    contact(c0 + (r - nj), which);
+                    contact(c0 + r, which);
                 }
             }
             __syncthreads();
@@ -5498,10 +5508,20 @@ static int32_t Check(cudaError_t e, const char* what)
 // resident at once, whose rows then stay in L2 across the passes.  Small
 // worlds get 128: four worlds share an SM instead of two, hiding each
 // other's joint chains, with one warp for a level's joint rows and three
-// for its contact rows.  Every variant keeps 128 registers per thread.
+// for its contact rows.  Every variant keeps 128 registers per thread
+// except the substep kernel of a single world and of a 256-thread class
+// of at most M3_SUBSTEP_ALONE_BLOCKS worlds an SM: a level has few rows a
+// block, each waiting for its own hundred words, and at up to 255
+// registers the words of a row are fetched at once where 128 spill and
+// fetch them in parts.  Measured (8 steps): one world of 210 boxes 2.24 ->
+// 1.80 ms, of 485 bodies 2.40 -> 1.99, 256 worlds of 100 hulls 2.13 ->
+// 1.84; the same change for all of 2,048 mixed worlds, where the second
+// block an SM hides the latency instead, 27.3 -> 30.2.
 // The split, each class's variant and its shared-memory budget form the
 // packing (m3gpu_set_packing, m3gpu_autotune_packing).
 #define M3_CLASSES 3
+#define M3_SUBSTEP_ALONE_BLOCKS 2
+static int32_t s_smCount = 148;
 static m3gpuPacking s_packing = {{769, 161},
                                  {512, 256, 128},
                                  {200 * 1024, M3_TWO_BLOCK_SMEM, 54 * 1024}};
@@ -5541,6 +5561,12 @@ static void LaunchClass(int32_t stage, int32_t c, cudaStream_t stream, const m3W
     }
     else if (c == 1)
     {
+        if (stage != 0 && count <= M3_SUBSTEP_ALONE_BLOCKS * s_smCount)
+        {
+            m3SubstepKernel<256, 1><<<count, 256, cacheBytes, stream>>>(views, order, count, dt,
+                                                                        substeps, cacheBytes);
+            return;
+        }
         M3_LAUNCH_CLASS(256, 2)
     }
     else
@@ -5572,6 +5598,10 @@ static int32_t SetClassSmem(int32_t c, int32_t bytes)
         if (e == cudaSuccess)
         {
             e = cudaFuncSetAttribute(m3SubstepKernel<256, 2>, a, bytes);
+        }
+        if (e == cudaSuccess)
+        {
+            e = cudaFuncSetAttribute(m3SubstepKernel<256, 1>, a, bytes);
         }
     }
     else
@@ -5964,7 +5994,6 @@ static void ClassStage(int32_t stage, const m3WorldView* views, const int32_t* o
 // Wide worlds: a single world with at least this many shape slots steps
 // its substep loop over a cooperative grid (m3WideSubstepKernel).
 static int32_t s_wideMinShapes = 4096;
-static int32_t s_smCount = 148;
 
 extern "C" int32_t m3gpu_set_wide_min_shapes(int32_t shapes)
 {
@@ -6146,7 +6175,7 @@ static void LaunchSolve(const m3WorldView* views, const int32_t* order, int32_t 
     }
     else if (classFirst == nullptr)
     {
-        m3SubstepKernel<256, 2><<<count, 256, cacheBytes>>>(views, order, count, dt, substeps,
+        m3SubstepKernel<256, 1><<<count, 256, cacheBytes>>>(views, order, count, dt, substeps,
                                                             cacheBytes);
     }
     else
