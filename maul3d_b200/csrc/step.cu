@@ -56,7 +56,6 @@
 // The wide kernels' grid: at most this many blocks, and the layout of the
 // wide prepare kernel's grid-shared words.
 #define M3_WIDE_MAX_BLOCKS 512
-#define M3_WW_FLAG 0        // 3 words: the colouring rounds' pending flags (round % 3)
 #define M3_WW_LEVELS 3      // joint levels
 #define M3_WW_CLEVELS 4     // contact levels
 #define M3_WW_JFLAG 5       // 3 words: the joint-level rounds' change flags (round % 3)
@@ -76,8 +75,7 @@
 // parallel rounds before the serial finish (one block per world; a wide
 // world's grid affords many more rounds).
 #define M3_COLOR_PENDING 0xFF
-#define M3_COLOR_ROUNDS 64
-#define M3_WIDE_COLOR_ROUNDS 4096
+#define M3_COLOR_ROUNDS 20
 // Rounds of the wide joint-level relaxation before the serial walk.
 #define M3_WIDE_JOINT_ROUNDS 4096
 
@@ -147,7 +145,7 @@ struct m3Scratch
     int32_t* movers;       // per body
     int32_t* moverFlag;    // per body
     uint32_t* bodyMask;    // per body
-    int32_t* colorMin;     // 2 per body: colouring round claims
+    int32_t* colorMin;     // 2 per body: colouring round claims, constraint list bounds
     m3StepPlan* plan;      // counts and offsets handed between the step kernels
     m3ConRows rows;        // contact rows, field-major, one slot per constraint
     int32_t* conPairIndex; // per constraint: its pair
@@ -2628,8 +2626,12 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3PrepareKernel(const m3WorldV
     // earliest uncoloured one on each of its bodies takes its colour at
     // once: exactly the masks the serial walk would see, and no two
     // constraints of a round touch the same body.  Each round colours
-    // at least the earliest uncoloured constraint; after M3_COLOR_ROUNDS
-    // rounds thread 0 finishes any rest in order.  Slots are then
+    // at least the earliest uncoloured constraint.  A world of loose bodies
+    // is done in a few rounds (two block barriers and two claims a
+    // constraint each); a stack's chain would take hundreds, so after
+    // M3_COLOR_ROUNDS rounds one warp finishes the rest in order (a
+    // pyramid of 210 boxes 114 -> 93 us a step; the warp from the start
+    // 77, but a world of 2,000 loose bodies 38 -> 81).  Slots are then
     // assigned colour by colour in constraint order (a stable counting
     // sort), as the serial list fill does.
     extern __shared__ __align__(16) uint8_t s_colorStage[];
@@ -2723,31 +2725,64 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3PrepareKernel(const m3WorldV
         }
         pendingLeft = __syncthreads_or(waiting) != 0;
     }
-    if (pendingLeft && tid == 0)
+    if (pendingLeft)
     {
-        // Long dependency chains: the rest in constraint order.
-        for (int32_t i = 0; i < constraintCount; ++i)
+        // Long dependency chains: one warp walks the rest in constraint
+        // order, 32 at a time.  A lane takes its colour when no earlier
+        // lane that shares a body with it is still uncoloured (the first
+        // uncoloured lane always may); which lanes share a body is found
+        // beforehand by all threads.
+        uint32_t* cEarlier = (uint32_t*)s.conLevel;
+        for (int32_t i = tid; i < constraintCount; i += NT)
         {
-            if (cColor[i] != M3_COLOR_PENDING)
+            uint32_t earlier = 0u;
+            if (cColor[i] == M3_COLOR_PENDING)
             {
-                continue;
+                const int2 p = cPair[i];
+                const int32_t i0 = i & ~31;
+                for (int32_t k = i0; k < i; ++k)
+                {
+                    const int2 q = cPair[k];
+                    const bool meets = (p.x >= 0 && (q.x == p.x || q.y == p.x)) ||
+                                       (p.y >= 0 && (q.x == p.y || q.y == p.y));
+                    earlier |= meets ? 1u << (k - i0) : 0u;
+                }
             }
-            const int2 p = cPair[i];
-            const uint32_t mask = (p.x >= 0 ? cMask[p.x] : 0u) | (p.y >= 0 ? cMask[p.y] : 0u);
-            int32_t color = __ffs((int)~mask) - 1;
-            color = color < M3_GRAPH_COLORS ? color : M3_GRAPH_COLORS;
-            cColor[i] = (uint8_t)color;
-            if (color < M3_GRAPH_COLORS)
+            cEarlier[i] = earlier;
+        }
+        __syncthreads();
+        for (int32_t i0 = 0; tid < 32 && i0 < constraintCount; i0 += 32)
+        {
+            const int32_t i = i0 + tid;
+            bool pending = i < constraintCount && cColor[i] == M3_COLOR_PENDING;
+            const int2 p = pending ? cPair[i] : make_int2(-1, -1);
+            const uint32_t earlier = pending ? cEarlier[i] : 0u;
+            uint32_t left = __ballot_sync(0xFFFFFFFFu, pending);
+            while (left != 0u)
             {
-                const uint32_t bit = 1u << color;
-                if (p.x >= 0)
+                if (pending && (earlier & left) == 0u)
                 {
-                    cMask[p.x] |= bit;
+                    const uint32_t mask =
+                        (p.x >= 0 ? cMask[p.x] : 0u) | (p.y >= 0 ? cMask[p.y] : 0u);
+                    int32_t color = __ffs((int)~mask) - 1;
+                    color = color < M3_GRAPH_COLORS ? color : M3_GRAPH_COLORS;
+                    cColor[i] = (uint8_t)color;
+                    if (color < M3_GRAPH_COLORS)
+                    {
+                        const uint32_t bit = 1u << color;
+                        if (p.x >= 0)
+                        {
+                            cMask[p.x] |= bit;
+                        }
+                        if (p.y >= 0)
+                        {
+                            cMask[p.y] |= bit;
+                        }
+                    }
+                    pending = false;
                 }
-                if (p.y >= 0)
-                {
-                    cMask[p.y] |= bit;
-                }
+                __syncwarp();
+                left = __ballot_sync(0xFFFFFFFFu, pending);
             }
         }
     }
@@ -3410,6 +3445,102 @@ __device__ int32_t GridExclusiveScan(int32_t* a, int32_t n, int32_t* ww, uint32_
     return total;
 }
 
+// The greedy colouring along the constraints' chains (every thread of a
+// cooperative grid calls it, whole warps together; no thread waits for
+// another).  A lane that has coloured a constraint takes one off the
+// counts of the two that follow it on its bodies; a count that reaches
+// zero makes the constraint the lane's, to colour next or, when both did,
+// to keep on the lane's stack (linked through `link`), from which idle
+// lanes of the warp are given.  The masks pass from lane to lane through
+// L2, each written before its follower's count is taken.  Bound by the
+// longest chain's round trips to L2 (about 1 us a constraint, where a
+// round over all constraints between two grid barriers took 5.5 us):
+// colouring and schedule of 100 towers, 60,615 rows, 2.15 -> 0.71 ms a
+// step; of 7,000 loose bodies, a few rounds, 0.106 -> 0.125.
+__device__ __forceinline__ void WideColourChains(int32_t count, int32_t gtid, int32_t gstride,
+                                                 const int32_t* starts, const int2* pairs,
+                                                 const int2* next, int32_t* waits, int32_t* link,
+                                                 uint32_t* masks, uint8_t* colors)
+{
+    const int32_t lane = (int32_t)(threadIdx.x & 31);
+    const uint32_t below = (1u << lane) - 1u;
+    for (int32_t i0 = gtid - lane; i0 < count; i0 += gstride)
+    {
+        const int32_t i = i0 + lane;
+        int32_t at = i < count && starts[i] != 0 ? i : -1;
+        int32_t top = -1;
+        while (__any_sync(0xFFFFFFFFu, at >= 0))
+        {
+            int32_t after = -1;
+            if (at >= 0)
+            {
+                const int2 p = __ldcg(&pairs[at]);
+                const int2 n = __ldcg(&next[at]);
+                const uint32_t maskA = p.x >= 0 ? __ldcg(&masks[p.x]) : 0u;
+                const uint32_t maskB = p.y >= 0 ? __ldcg(&masks[p.y]) : 0u;
+                // First clear bit among the 16 colours; 16 = overflow.
+                int32_t color = __ffs((int)~(maskA | maskB)) - 1;
+                color = color < M3_GRAPH_COLORS ? color : M3_GRAPH_COLORS;
+                colors[at] = (uint8_t)color;
+                const uint32_t bit = color < M3_GRAPH_COLORS ? 1u << color : 0u;
+                if (p.x >= 0)
+                {
+                    __stcg(&masks[p.x], maskA | bit);
+                }
+                if (p.y >= 0)
+                {
+                    __stcg(&masks[p.y], maskB | bit);
+                }
+                __threadfence();
+                const int32_t leftA = n.x >= 0 ? atomicSub(&waits[n.x], 1) : 0;
+                const int32_t leftB = n.y >= 0 ? atomicSub(&waits[n.y], 1) : 0;
+                __threadfence();
+                after = leftA == 1 ? n.x : -1;
+                if (leftB == 1)
+                {
+                    if (after >= 0)
+                    {
+                        link[n.y] = top;
+                        top = n.y;
+                    }
+                    else
+                    {
+                        after = n.y;
+                    }
+                }
+            }
+            if (after < 0 && top >= 0)
+            {
+                after = top;
+                top = link[top];
+            }
+            at = after;
+            // The k-th idle lane takes the top of the k-th lane that has
+            // one to spare.
+            const uint32_t idle = __ballot_sync(0xFFFFFFFFu, at < 0);
+            const uint32_t spare = __ballot_sync(0xFFFFFFFFu, top >= 0);
+            if (idle != 0u && spare != 0u)
+            {
+                const int32_t given = top;
+                const int32_t rank = __popc((at < 0 ? idle : spare) & below);
+                const int32_t moves = min(__popc(idle), __popc(spare));
+                const int32_t giver = at < 0 && rank < moves ? (int32_t)__fns(spare, 0, rank + 1)
+                                                             : lane;
+                const int32_t taken = __shfl_sync(0xFFFFFFFFu, given, giver);
+                if (at < 0)
+                {
+                    at = rank < moves ? taken : -1;
+                }
+                else if (top >= 0 && rank < moves)
+                {
+                    top = link[top];
+                }
+                __syncwarp();
+            }
+        }
+    }
+}
+
 // The preparation of one wide world over a cooperative grid: the same
 // stages, in the same order and with the same arithmetic, as
 // m3PrepareKernel's (islands and wake, contact and joint selection, joint
@@ -3779,22 +3910,26 @@ __global__ void __launch_bounds__(NT, 2) m3WidePrepareKernel(const m3WorldView* 
     M3_WIDE_MARK(M3_PHASE_PREPARE)
 
     // Greedy 16-colour first-free-bit colouring in constraint order, the
-    // overflow bucket last (solver.c:2750-2810), in rounds: each round
-    // colours every uncoloured constraint that is the earliest
-    // uncoloured one on each of its awake dynamic bodies (exactly the
-    // masks the serial walk sees); after M3_COLOR_ROUNDS rounds one
-    // thread finishes the rest in order.
+    // overflow bucket last (solver.c:2750-2810).  A constraint's colour
+    // depends only on the colours of the earlier constraints that share
+    // one of its awake dynamic bodies, so each constraint waits for the
+    // latest earlier one on each body and is followed by the next one on
+    // each: whoever colours the last it waited for colours it next
+    // (WideColourChains), without a barrier on the way.
     uint32_t* cMask = s.bodyMask;
-    int32_t* cMin0 = s.colorMin;
-    int32_t* cMin1 = s.colorMin + sc->bodyCap;
+    int32_t* conFirst = s.colorMin;               // per body: its constraints' start
+    int32_t* conEnd = s.colorMin + sc->bodyCap;   // per body: and end
+    int32_t* conAdj = (int32_t*)s.rows.ro;        // (the rows are written after this kernel)
+    int2* conNext = (int2*)(conAdj + 2 * (int64_t)constraintCount);
+    int32_t* conWaits = (int32_t*)(conNext + constraintCount);
     int2* cPair = s.conPair;
     uint8_t* cColor = s.colors;
     for (int32_t i = gtid; i < bodyMax; i += gstride)
     {
         cMask[i] = 0u;
-        cMin0[i] = INT32_MAX;
-        cMin1[i] = INT32_MAX;
+        conFirst[i] = 0;
     }
+    M3_GSYNC()
     for (int32_t i = gtid; i < constraintCount; i += gstride)
     {
         const uint64_t key = keys[s.conPairIndex[i]];
@@ -3803,121 +3938,66 @@ __global__ void __launch_bounds__(NT, 2) m3WidePrepareKernel(const m3WorldView* 
         const int32_t a = w.btype[bodyA] == M3_BODY_DYNAMIC && w.awake[bodyA] ? bodyA : -1;
         const int32_t b = w.btype[bodyB] == M3_BODY_DYNAMIC && w.awake[bodyB] ? bodyB : -1;
         cPair[i] = make_int2(a, b);
-        cColor[i] = M3_COLOR_PENDING;
-    }
-    if (lead)
-    {
-        ww[M3_WW_FLAG] = 0;
-        ww[M3_WW_FLAG + 1] = 0;
-        ww[M3_WW_FLAG + 2] = 0;
+        if (a >= 0)
+        {
+            atomicAdd(&conFirst[a], 1);
+        }
+        if (b >= 0)
+        {
+            atomicAdd(&conFirst[b], 1);
+        }
     }
     M3_GSYNC()
-    // Round r raises flag r % 3 and every block reads it after the round's
-    // last barrier; it is cleared again at the start of round r + 2, after
-    // two more barriers, when no block can still be reading it.
-    bool pendingLeft = constraintCount > 0;
-    for (int32_t round = 0; pendingLeft && round < M3_WIDE_COLOR_ROUNDS; ++round)
+    if (GridExclusiveScan<NT>(conFirst, bodyMax, ww, bar) < 0)
     {
-        int32_t* cur = (round & 1) ? cMin1 : cMin0;
-        int32_t* nxt = (round & 1) ? cMin0 : cMin1;
-        if (lead)
-        {
-            ww[M3_WW_FLAG + (round + 1) % 3] = 0; // the next round's flag
-        }
-        for (int32_t i = gtid; i < constraintCount; i += gstride)
-        {
-            if (cColor[i] == M3_COLOR_PENDING)
-            {
-                const int2 p = cPair[i];
-                if (p.x >= 0)
-                {
-                    atomicMin(&cur[p.x], i);
-                }
-                if (p.y >= 0)
-                {
-                    atomicMin(&cur[p.y], i);
-                }
-            }
-        }
-        M3_GSYNC()
-        bool waiting = false;
-        for (int32_t i = gtid; i < constraintCount; i += gstride)
-        {
-            if (cColor[i] != M3_COLOR_PENDING)
-            {
-                continue;
-            }
-            const int2 p = cPair[i];
-            const bool ready = (p.x < 0 || cur[p.x] == i) && (p.y < 0 || cur[p.y] == i);
-            if (p.x >= 0)
-            {
-                nxt[p.x] = INT32_MAX;
-            }
-            if (p.y >= 0)
-            {
-                nxt[p.y] = INT32_MAX;
-            }
-            if (!ready)
-            {
-                waiting = true;
-                continue;
-            }
-            const uint32_t mask = (p.x >= 0 ? cMask[p.x] : 0u) | (p.y >= 0 ? cMask[p.y] : 0u);
-            int32_t color = __ffs((int)~mask) - 1;
-            color = color < M3_GRAPH_COLORS ? color : M3_GRAPH_COLORS;
-            cColor[i] = (uint8_t)color;
-            if (color < M3_GRAPH_COLORS)
-            {
-                const uint32_t bit = 1u << color;
-                if (p.x >= 0)
-                {
-                    cMask[p.x] |= bit;
-                }
-                if (p.y >= 0)
-                {
-                    cMask[p.y] |= bit;
-                }
-            }
-        }
-        if (waiting)
-        {
-            ww[M3_WW_FLAG + round % 3] = 1;
-        }
-        M3_GSYNC()
-        pendingLeft = vww[M3_WW_FLAG + round % 3] != 0;
+        return;
     }
-    if (pendingLeft)
+    for (int32_t i = gtid; i < bodyMax; i += gstride)
     {
-        if (lead)
-        {
-            for (int32_t i = 0; i < constraintCount; ++i)
-            {
-                if (cColor[i] != M3_COLOR_PENDING)
-                {
-                    continue;
-                }
-                const int2 p = cPair[i];
-                const uint32_t mask =
-                    (p.x >= 0 ? cMask[p.x] : 0u) | (p.y >= 0 ? cMask[p.y] : 0u);
-                int32_t color = __ffs((int)~mask) - 1;
-                color = color < M3_GRAPH_COLORS ? color : M3_GRAPH_COLORS;
-                cColor[i] = (uint8_t)color;
-                if (color < M3_GRAPH_COLORS)
-                {
-                    const uint32_t bit = 1u << color;
-                    if (p.x >= 0)
-                    {
-                        cMask[p.x] |= bit;
-                    }
-                    if (p.y >= 0)
-                    {
-                        cMask[p.y] |= bit;
-                    }
-                }
-            }
-        }
-        M3_GSYNC()
+        conEnd[i] = conFirst[i];
     }
+    M3_GSYNC()
+    for (int32_t i = gtid; i < constraintCount; i += gstride)
+    {
+        const int2 p = cPair[i];
+        if (p.x >= 0)
+        {
+            conAdj[atomicAdd(&conEnd[p.x], 1)] = i;
+        }
+        if (p.y >= 0)
+        {
+            conAdj[atomicAdd(&conEnd[p.y], 1)] = i;
+        }
+    }
+    M3_GSYNC()
+    for (int32_t i = gtid; i < constraintCount; i += gstride)
+    {
+        const int2 p = cPair[i];
+        int32_t waits = 0;
+        const auto follow = [&](int32_t body) {
+            int32_t next = INT32_MAX;
+            bool earlier = false;
+            for (int32_t k = body >= 0 ? conFirst[body] : 0; body >= 0 && k < conEnd[body]; ++k)
+            {
+                const int32_t o = conAdj[k];
+                earlier = earlier || o < i;
+                next = o > i && o < next ? o : next;
+            }
+            waits += earlier ? 1 : 0;
+            return next == INT32_MAX ? -1 : next;
+        };
+        const int32_t nextA = follow(p.x);
+        const int32_t nextB = follow(p.y);
+        conNext[i] = make_int2(nextA, nextB);
+        conWaits[i] = waits;
+        // Chains start at the constraints that wait for none; the array
+        // below is free once the lists are read.
+        s.conLevel[i] = waits == 0 ? 1 : 0;
+    }
+    M3_GSYNC()
+    WideColourChains(constraintCount, gtid, gstride, s.conLevel, cPair, conNext, conWaits, conAdj,
+                     cMask, cColor);
+    M3_GSYNC()
     // Slots: colour by colour, constraint order inside a colour (a stable
     // counting sort).  Each block owns a contiguous range of constraints:
     // its count per colour, then its first slot per colour, then its
@@ -4019,7 +4099,7 @@ __global__ void __launch_bounds__(NT, 2) m3WidePrepareKernel(const m3WorldView* 
     // the last joint level on either of its awake dynamic bodies and one
     // past the level of the previous contact (colour order) on either of
     // them; the overflow colour stays last and serial.
-    int32_t* cLast = cMin0;
+    int32_t* cLast = s.colorMin;
     for (int32_t i = gtid; i < bodyMax; i += gstride)
     {
         cLast[i] = jointCount > 0 ? s.ready[i] + 1 : 0;
