@@ -6466,62 +6466,108 @@ static uint64_t RecordTreeLaunch(cudaStream_t stream)
 // The tree launches of a call read their own copy of the call's world
 // table: they finish behind the call, after the next call may have
 // rebuilt the batch table.  A copy is reused (oldest first) once the
-// last launch reading it is done.
-#define M3_TREE_TABLES 8
+// last launch reading it is done.  With as many copies as half the
+// ring's steps, a call neither waits for a copy nor for the ring before
+// M3_TREE_LAG steps are behind.
+#define M3_TREE_TABLES (M3_TREE_LAG - M3_TREE_REPLAY_AT)
 struct m3TreeTable
 {
     m3WorldView* views = nullptr;
     int32_t* order = nullptr;
     int32_t* steps = nullptr;     // per world: recorded steps to replay
     int32_t* hostSteps = nullptr; // page-locked staging of `steps`
-    int32_t cap = 0;
     uint64_t lastSeq = 0;
 };
 static m3TreeTable s_treeTables[M3_TREE_TABLES];
 static int32_t s_treeTableNext = 0;
+static int32_t s_treeTableCap = 0;        // worlds every copy has room for
+static uint8_t* s_treeTableDev = nullptr; // the copies, one allocation
+static int32_t* s_treeTableHost = nullptr;
+
+static int32_t WaitTreeTable(m3TreeTable* t)
+{
+    if (t->lastSeq != 0)
+    {
+        const cudaError_t e = cudaEventSynchronize(TreeEventFor(t->lastSeq));
+        if (e != cudaSuccess)
+        {
+            return m3gpuSetError(M3GPU_ERR_CUDA, "tree table: %s", cudaGetErrorString(e));
+        }
+        t->lastSeq = 0;
+    }
+    return M3GPU_OK;
+}
+
+// Room for `count` worlds in every copy.
+static int32_t GrowTreeTables(int32_t count)
+{
+    for (m3TreeTable& t : s_treeTables)
+    {
+        const int32_t rc = WaitTreeTable(&t);
+        if (rc != M3GPU_OK)
+        {
+            return rc;
+        }
+    }
+    cudaFree(s_treeTableDev);
+    cudaFreeHost(s_treeTableHost);
+    s_treeTableDev = nullptr;
+    s_treeTableHost = nullptr;
+    s_treeTableCap = 0;
+    const size_t viewBytes = (size_t)m3AlignUp((int64_t)sizeof(m3WorldView) * count, 256);
+    const size_t wordBytes = (size_t)m3AlignUp((int64_t)sizeof(int32_t) * count, 256);
+    const size_t bytes = viewBytes + 2 * wordBytes;
+    cudaError_t e = cudaMalloc((void**)&s_treeTableDev, bytes * M3_TREE_TABLES);
+    if (e == cudaSuccess)
+    {
+        e = cudaMallocHost((void**)&s_treeTableHost, wordBytes * M3_TREE_TABLES);
+    }
+    if (e != cudaSuccess)
+    {
+        return m3gpuSetError(M3GPU_ERR_CUDA, "tree table: %s", cudaGetErrorString(e));
+    }
+    for (int32_t k = 0; k < M3_TREE_TABLES; ++k)
+    {
+        m3TreeTable& t = s_treeTables[k];
+        uint8_t* base = s_treeTableDev + bytes * (size_t)k;
+        t.views = (m3WorldView*)base;
+        t.order = (int32_t*)(base + viewBytes);
+        t.steps = (int32_t*)(base + viewBytes + wordBytes);
+        t.hostSteps = (int32_t*)((uint8_t*)s_treeTableHost + wordBytes * (size_t)k);
+    }
+    s_treeTableCap = count;
+    return M3GPU_OK;
+}
+
+// Whether the next copy can be taken without waiting (also when an
+// earlier error stands, which taking it then reports).
+static bool TreeTableFree()
+{
+    const m3TreeTable& t = s_treeTables[s_treeTableNext];
+    if (t.lastSeq == 0 || cudaPeekAtLastError() != cudaSuccess)
+    {
+        return true;
+    }
+    if (cudaEventQuery(TreeEventFor(t.lastSeq)) == cudaErrorNotReady)
+    {
+        cudaGetLastError(); // not an error
+        return false;
+    }
+    return true;
+}
 
 static int32_t TakeTreeTable(int32_t count, m3TreeTable** out)
 {
     m3TreeTable& t = s_treeTables[s_treeTableNext];
     s_treeTableNext = (s_treeTableNext + 1) % M3_TREE_TABLES;
-    if (t.lastSeq != 0)
+    int32_t rc = WaitTreeTable(&t);
+    if (rc == M3GPU_OK && count > s_treeTableCap)
     {
-        const cudaError_t e = cudaEventSynchronize(TreeEventFor(t.lastSeq));
-        if (e != cudaSuccess)
-        {
-            return m3gpuSetError(M3GPU_ERR_CUDA, "tree table: %s", cudaGetErrorString(e));
-        }
-        t.lastSeq = 0;
+        rc = GrowTreeTables(count);
     }
-    if (count > t.cap)
+    if (rc != M3GPU_OK)
     {
-        cudaFree(t.views);
-        cudaFree(t.order);
-        cudaFree(t.steps);
-        cudaFreeHost(t.hostSteps);
-        t.views = nullptr;
-        t.order = nullptr;
-        t.steps = nullptr;
-        t.hostSteps = nullptr;
-        t.cap = 0;
-        cudaError_t e = cudaMalloc((void**)&t.views, sizeof(m3WorldView) * (size_t)count);
-        if (e == cudaSuccess)
-        {
-            e = cudaMalloc((void**)&t.order, sizeof(int32_t) * (size_t)count);
-        }
-        if (e == cudaSuccess)
-        {
-            e = cudaMalloc((void**)&t.steps, sizeof(int32_t) * (size_t)count);
-        }
-        if (e == cudaSuccess)
-        {
-            e = cudaMallocHost((void**)&t.hostSteps, sizeof(int32_t) * (size_t)count);
-        }
-        if (e != cudaSuccess)
-        {
-            return m3gpuSetError(M3GPU_ERR_CUDA, "tree table: %s", cudaGetErrorString(e));
-        }
-        t.cap = count;
+        return rc;
     }
     // Ordered on the default stream after the batch table's upload and
     // before the broadphase the tree launches wait for.
@@ -6840,10 +6886,10 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
         cudaEventRecord(ev[1]);
         if (anyTracked)
         {
-            // The step's moves are recorded; once M3_TREE_REPLAY_AT steps
-            // wait in a world's ring, the batch's recorded steps are
-            // replayed on the tree's stream beside the following steps.
-            bool replay = false;
+            // The step's moves are recorded; the batch's recorded steps
+            // are replayed on the tree's stream beside the rest of the
+            // step and the following ones.
+            bool replay = TreeTableFree();
             for (m3HostWorld* w : tracked)
             {
                 w->treeSlotSeq[(w->treeFirst + w->treeCount) % M3_TREE_LAG] = 0;
