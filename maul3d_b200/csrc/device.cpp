@@ -870,9 +870,7 @@ extern "C" int32_t m3gpu_slot_save(m3WorldId world, int32_t slot)
     }
     m3gpuWaitTree(w);
     const size_t bytes = (size_t)w->persistentBytes;
-    rc = CudaCheck(cudaMemcpyAsync(w->dslots + bytes * (size_t)slot, w->dslab, bytes,
-                                   cudaMemcpyDeviceToDevice, 0),
-                   "save device snapshot slot");
+    rc = m3gpuLaunchSlotCopy(w->dslots + bytes * (size_t)slot, w->dslab, (int64_t)bytes);
     if (rc != M3GPU_OK)
     {
         return rc;
@@ -910,9 +908,7 @@ extern "C" int32_t m3gpu_slot_restore(m3WorldId world, int32_t slot)
     // Replays of the current timeline write the slab: they finish first.
     m3gpuWaitTree(w);
     const size_t bytes = (size_t)w->persistentBytes;
-    rc = CudaCheck(cudaMemcpyAsync(w->dslab, w->dslots + bytes * (size_t)slot, bytes,
-                                   cudaMemcpyDeviceToDevice, 0),
-                   "restore device snapshot slot");
+    rc = m3gpuLaunchSlotCopy(w->dslab, w->dslots + bytes * (size_t)slot, (int64_t)bytes);
     if (rc != M3GPU_OK)
     {
         return rc;

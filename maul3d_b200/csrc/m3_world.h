@@ -60,6 +60,9 @@ struct m3UploadItem
     int32_t pad;
 };
 int32_t m3gpuLaunchUpload(const m3UploadItem* items, int32_t count);
+// Copies a world's state (a multiple of 16 bytes, as its slab's layout
+// makes it) on the default stream (upload.cu).
+int32_t m3gpuLaunchSlotCopy(uint8_t* dst, const uint8_t* src, int64_t bytes);
 // Bytes of one hull slab an upload copies (the parts its counts use).
 int64_t m3HullUsedBytes(const m3HullData* h);
 // Content key of an interned hull slab for the dedup index: FNV-1a over
