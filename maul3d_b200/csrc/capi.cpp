@@ -407,8 +407,9 @@ extern "C" int32_t m3gpu_autotune_packing(const m3WorldId* worlds, int32_t count
     int32_t done = 0;
     // One real step under packing `p`; its prepare and substep stages'
     // device time in *ms.  The broadphase trees' pending moves are
-    // replayed first, untimed: a replay launched beside the step (every
-    // 16 steps) would share the SMs with it and slow the stages timed.
+    // replayed first, untimed, and the step's own wait for a later step
+    // or reader: a replay beside the step would share the SMs with it and
+    // slow the stages timed.
     auto measure = [&](const m3gpuPacking& p, float* ms) -> int32_t {
         int32_t r = m3gpu_flush_trees(worlds, count);
         if (r == M3GPU_OK)
@@ -417,7 +418,7 @@ extern "C" int32_t m3gpu_autotune_packing(const m3WorldId* worlds, int32_t count
         }
         if (r == M3GPU_OK)
         {
-            r = m3gpuStepBatch(ws.data(), count, dt, substeps, 1);
+            r = m3gpuStepBatch(ws.data(), count, dt, substeps, 1, nullptr, 0, false);
         }
         if (r != M3GPU_OK)
         {

@@ -427,9 +427,11 @@ void m3gpuDeviceHits(const m3HostWorld* w, const uint8_t** flags, const m3HitEve
 // Step and hash entry points (step.cu).
 // `ops` (optional) are body commands applied on the device before the
 // first step: m3BodyOp.world indexes `worlds`; per world they apply in
-// array order.
+// array order.  Without `replay` the steps' tree moves wait in the ring for
+// a later step or reader.
 int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t substeps,
-                       int32_t steps, const struct m3BodyOp* ops = nullptr, int32_t opCount = 0);
+                       int32_t steps, const struct m3BodyOp* ops = nullptr, int32_t opCount = 0,
+                       bool replay = true);
 int32_t m3gpuHashBatch(m3HostWorld** worlds, int32_t count, uint64_t* out);
 // Orders the default stream after every tree launch still pending for
 // the world (step.cu): anything that reads or overwrites its tree or its

@@ -4,23 +4,30 @@
 // Launches per step:
 //   m3BroadKernel        one block per world: fresh bounds, sort-and-sweep
 //                        and the canonical (sorted) pair list;
+//   m3TreeKernel         the step's tree moves, on a stream of its own
+//                        beside everything below and the following steps;
 //   m3PairOffsetsKernel  prefix of the worlds' pair counts;
 //   m3FamilyCount/ScatterKernel  bucket the batch's flattened pairs by
 //                        pair family;
 //   m3NarrowFamilyKernel<F>  one per covered family, one thread per pair
 //                        of its bucket: the narrowphase with the
-//                        warm-start carry (m3NarrowKernel, all families
-//                        in one, serves the single-world path);
+//                        warm-start carry (m3NarrowTerrainKernel<F>, a
+//                        group of lanes per pair, for capsules and hulls
+//                        on heightfields; m3NarrowKernel, all families in
+//                        one, for a few small worlds);
 //   m3PrepareKernel      one block per world: islands and wake, contact
 //                        selection, graph colouring, contact rows written
 //                        into their solve slots, joint rows and their
 //                        dependency levels, movers;
 //   m3SubstepKernel      one block per world: the substep loop (integrate,
-//                        warm start, colour-by-colour solve, integrate
+//                        warm start, level-by-level solve, integrate
 //                        positions, relax) with body velocities in shared
 //                        memory, restitution and the impulse store;
 //   m3FinishKernel       one block per world: the continuous pass against
 //                        planes, the sleep pass and the step counter.
+// One large world alone takes the m3Wide* kernels instead, every stage
+// over the whole grid, and the m3Island* kernels for its substep loop when
+// its islands fit a block each.
 // Block barriers separate every dependent phase, so inside a world the
 // order of every write is the reference's; across worlds nothing is
 // shared.  Worlds are ordered largest first so the long worlds start
@@ -6739,7 +6746,7 @@ extern "C" int32_t m3gpu_flush_trees(const m3WorldId* worldIds, int32_t count)
 }
 
 int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t substeps,
-                       int32_t steps, const m3BodyOp* ops, int32_t opCount)
+                       int32_t steps, const m3BodyOp* ops, int32_t opCount, bool replayBeside)
 {
     M3_DEVICE_GUARD;
     int32_t rc = m3gpuEnsureDevice();
@@ -6889,7 +6896,7 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
             // The step's moves are recorded; the batch's recorded steps
             // are replayed on the tree's stream beside the rest of the
             // step and the following ones.
-            bool replay = TreeTableFree();
+            bool replay = replayBeside && TreeTableFree();
             for (m3HostWorld* w : tracked)
             {
                 w->treeSlotSeq[(w->treeFirst + w->treeCount) % M3_TREE_LAG] = 0;
