@@ -530,7 +530,8 @@ def serving_run(m3, distinct: int, seed: int, rates: list[float], budget: int,
                         ("prepareMs", "admitMs", "stepMs", "retireMs", "waitMs")},
             "workers": stats["workers"]})
     out["same_answer_every_time"] = mismatched_runs == 0
-    if cpu_baseline:
+    from oracle import ref
+    if cpu_baseline and ref.build():
         threads = os.cpu_count() or 1
         secs, ref_hashes = reference_serving(raw, caps, threads)
         mism = sum(1 for i in range(distinct) if served.get(i) != ref_hashes[i])
@@ -963,7 +964,8 @@ def main() -> None:
         singles = {spec[0]: single_world_run(m3, args, spec) for spec in SINGLE_WORLDS
                    if spec[0] in want}
     terrain = None
-    if rank == 0 and args.terrain_worlds > 0 and not args.no_cpu_baseline:
+    from oracle import ref
+    if rank == 0 and args.terrain_worlds > 0 and not args.no_cpu_baseline and ref.build():
         terrain = terrain_run(m3, args, rank_seed + 91)
 
     if rank == 0:
