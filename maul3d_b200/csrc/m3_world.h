@@ -157,18 +157,20 @@ struct m3StepProfile
 
 // The broadphase tree is state only snapshots read: each step records
 // its leaf moves in a ring of this many per-step lists in the world's
-// scratch, and the moves are replayed into the tree beside the rest of
-// the step and the following ones, on the tree's own stream: after every
-// step while a table for the launch is free, else once M3_TREE_REPLAY_AT
-// steps have gathered, when the ring would overflow, or at once when
-// something reads or overwrites the tree.  A step's replay is a chain of
-// its own and takes little of the GPU, so it starts as early as it can:
-// eight steps of a 485-body world and its tree 10.3 -> 7.3 ms, of 64
-// worlds of up to 2,000 bodies 29.6 -> 23.1, of 2,048 worlds 98 -> 90
-// against gathering 16 steps first; 64 steps of 1,024 100-body worlds in
-// one call, where the launches hide nothing, 97 -> 98 ms.
+// scratch, and the moves are replayed into the tree on the tree's own
+// stream, beside the rest of the step and the following ones: after every
+// step for a batch of at most M3_TREE_EARLY_WORLDS worlds an SM while a
+// table for the launch is free, else once M3_TREE_REPLAY_AT steps have
+// gathered, when the ring would overflow, or at once when something reads
+// or overwrites the tree.  A replay is a chain of its own and takes little
+// of a GPU that has room: eight steps of a 485-body world and its tree 10.3
+// -> 7.3 ms, of 64 worlds of up to 2,000 bodies 29.6 -> 23.1, of 2,048
+// worlds 98 -> 90 against gathering first.  4,096 worlds fill the GPU:
+// steps and trees together take as long either way (64 steps 386 -> 384
+// ms), and a step whose tree nobody reads yet 12.2 -> 15.2.
 #define M3_TREE_LAG 32
 #define M3_TREE_REPLAY_AT 16
+#define M3_TREE_EARLY_WORLDS 16
 
 struct m3HostWorld
 {

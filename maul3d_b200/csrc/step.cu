@@ -6896,7 +6896,8 @@ int32_t m3gpuStepBatch(m3HostWorld** worlds, int32_t count, float dt, int32_t su
             // The step's moves are recorded; the batch's recorded steps
             // are replayed on the tree's stream beside the rest of the
             // step and the following ones.
-            bool replay = replayBeside && TreeTableFree();
+            bool replay = replayBeside && count <= M3_TREE_EARLY_WORLDS * s_smCount &&
+                          TreeTableFree();
             for (m3HostWorld* w : tracked)
             {
                 w->treeSlotSeq[(w->treeFirst + w->treeCount) % M3_TREE_LAG] = 0;

@@ -36,3 +36,21 @@ def test_one_call_single_calls_and_flushes_agree(m3, spec, count, steps):
     finally:
         for w in together + single + flushed:
             w.destroy()
+
+
+@pytest.mark.parametrize("count", [16 * 148, 16 * 148 + 1])
+def test_batches_about_the_early_line(m3, count):
+    worlds = [m3.World.scene(SCENE_UNEVEN, 1 + i % 3, 6) for i in range(count)]
+    alone = [m3.World.scene(SCENE_UNEVEN, 1 + i, 6) for i in range(3)]
+    try:
+        for steps in (3, 18):
+            m3.step_worlds(worlds, DT, 2, steps)
+            expected = []
+            for w in alone:
+                w.step(DT, 2, steps)
+                expected.append(m3.snapshot(w))
+            for i in (0, 1, 2, count - 3, count - 2, count - 1):
+                assert m3.snapshot(worlds[i]) == expected[i % 3]
+    finally:
+        for w in worlds + alone:
+            w.destroy()
