@@ -1014,7 +1014,10 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
     {
         pow2 <<= 1;
     }
-    uint64_t* elems = pow2 <= sortCap ? s_sort : s.sortKey;
+    // Where the elements lie is decided here for the whole sort, by the
+    // slots: fewer of them may be swept (planes, dead slots).
+    const bool inShared = pow2 <= sortCap;
+    uint64_t* elems = inShared ? s_sort : s.sortKey;
     for (int32_t i = tid; i < shapeMax; i += NT)
     {
         s.rowCount[i] = 0;
@@ -1104,7 +1107,7 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3BroadKernel(const m3WorldVie
         elems[i] = M3_SWEEP_NONE;
     }
     __syncthreads();
-    if (pow2 <= sortCap)
+    if (inShared)
     {
         BlockSort<NT>(s_sort, pow2);
     }
