@@ -693,15 +693,17 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
     m3Scratch s;
     ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap, treeLag);
     const int32_t tail = sc->treeTail;
-    const bool refused = sc->status != 0;
-    __syncthreads();
+    // A refused world's tree is not kept (its state is unspecified after
+    // a refusal).  The step's kernels run beside this one and may refuse
+    // the world at any moment, so one thread's reading decides for the
+    // block: a walker without its staging warp would walk chunks that
+    // nobody staged.
+    const bool refused = __syncthreads_or(threadIdx.x == 0 && sc->status != 0) != 0;
     if (threadIdx.x == 0)
     {
         sc->treeTail = tail + n;
         s_stop = 0;
     }
-    // A refused world's tree is not kept (its state is unspecified after
-    // a refusal).
     if (refused)
     {
         return;
