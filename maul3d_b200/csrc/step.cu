@@ -689,7 +689,6 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
         return;
     }
     __shared__ m3TreeChunk chunks[2];
-    __shared__ int32_t s_stop;
     m3Scratch s;
     ScratchCarve(&s, w.scratch, sc->bodyCap, sc->shapeCap, sc->jointCap, sc->pairCap, treeLag);
     const int32_t tail = sc->treeTail;
@@ -702,7 +701,6 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
     if (threadIdx.x == 0)
     {
         sc->treeTail = tail + n;
-        s_stop = 0;
     }
     if (refused)
     {
@@ -742,10 +740,11 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
     {
         const m3TreeChunk& chunk = chunks[c];
         const int32_t moves = chunk.count;
-        if (moves == 0 || s_stop != 0)
+        if (moves == 0)
         {
             break;
         }
+        int32_t stop = 0;
         if (!walker)
         {
             m3StageTreeChunk(w, s, tail, n, treeLag, &at, &chunks[c ^ 1], lane);
@@ -753,7 +752,6 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
         else
         {
             tree.tracked = tree.tracked && chunk.plain != 0;
-            int32_t stop = 0;
             for (int32_t m = 0; m < moves && stop == 0; ++m)
             {
                 const int32_t leaf = chunk.leaf[m];
@@ -771,11 +769,14 @@ __global__ void __launch_bounds__(M3_TREE_THREADS)
                 {
                     sc->statusDetail = 6001;
                 }
-                s_stop = 1;
             }
             total += moves;
         }
-        __syncthreads();
+        // Both warps leave together, at the barrier.
+        if (__syncthreads_or(stop != 0) != 0)
+        {
+            break;
+        }
     }
     if (!walker)
     {

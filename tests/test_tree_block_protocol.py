@@ -4,8 +4,9 @@ m3TreeKernel's text is taken from the source and compiled for the host
 with a thread in place of each warp (lane 0 of the walking and of the
 staging one), plain stand-ins for the tree, the staging and the scratch,
 and a barrier that notices a warp arriving after the other has left the
-kernel.  The stand-ins choose the schedule that decides: a world refused
-by the step's kernels between the two warps' reads of its status.
+kernel.  The stand-ins choose the schedules that decide: a world refused
+by the step's kernels between the two warps' reads of its status, and a
+walk that ends at a malformed tree while the staging warp is late.
 """
 import re
 import shutil
@@ -205,3 +206,9 @@ def test_a_refusal_between_the_warps_reads(replay, scenario):
     lone, unstaged, moved, _ = replay(scenario)
     assert (lone, unstaged) == (0, 0)
     assert moved in (0, 96)
+
+
+def test_a_malformed_tree_ends_both_warps_at_the_barrier(replay):
+    lone, unstaged, moved, status = replay(3)
+    assert (lone, unstaged) == (0, 0)
+    assert (moved, status) == (40, 3)
