@@ -808,8 +808,9 @@ def main() -> None:
     ms = e0.elapsed_time(e1)
     stage_ms = m3.kernel_ms()
     # The broadphase trees are snapshot state, replayed from the recorded
-    # leaf moves when read (or every 16 steps): the catch-up of whatever
-    # the timed steps left unreplayed, timed on its own.
+    # leaf moves beside the steps (after each step, or 16 at a time in a
+    # batch of more than 16 worlds an SM) or when read: the catch-up of
+    # whatever the timed steps left unreplayed, timed on its own.
     t0 = time.perf_counter()
     m3.flush_trees(worlds)
     tree_catchup_ms = (time.perf_counter() - t0) * 1e3
@@ -990,7 +991,8 @@ def main() -> None:
                                     "baseline_ms": round(t["baseline_ms"], 3),
                                     "adopted": t["adopted"]} for t in trials]},
             "tree": {"note": "the broadphase tree (snapshot state) replays recorded leaf moves "
-                             "every 16 steps beside the steps, or when read; catchup_ms = "
+                             "beside the steps (after each step; 16 steps at a time in a batch "
+                             "of more than 16 worlds an SM) or when read; catchup_ms = "
                              "replaying what the timed steps left, after them",
                      "catchup_ms": tree_catchup_ms,
                      "value_with_catchup": total_bs / ((ms_max + tree_catchup_ms) / 1000.0)},
