@@ -79,9 +79,9 @@ SCENE_TERRAIN = 5
 # three size classes; the 4th step from creation) on the default
 # workload, from ncu (dram__bytes_read.sum + dram__bytes_write.sum, one
 # pass; profiles/m3SubstepKernel_uneven4096.txt gives the command):
-# 902.5 + 677.7 MB (512-thread class), 381.8 + 391.5 MB (256), 80.5 +
-# 102.4 MB (128).  Reported for that workload only.
-SUBSTEP_TRAFFIC_DEFAULT = (902.5 + 677.7 + 381.8 + 391.5 + 80.5 + 102.4) * 1e6
+# 1108.5 + 746.9 MB (512-thread class), 437.6 + 418.6 MB (256), 85.1 +
+# 117.3 MB (128).  Reported for that workload only.
+SUBSTEP_TRAFFIC_DEFAULT = (1108.5 + 746.9 + 437.6 + 418.6 + 85.1 + 117.3) * 1e6
 BYTES_PER_MOVER_SUBSTEP = 314
 BYTES_PER_CONTACT_SUBSTEP = 3 * (456 + 2 * 48 + 2 * 28)
 BYTES_PER_JOINT_SUBSTEP = 3 * (472 + 152)
