@@ -5088,6 +5088,26 @@ __device__ __noinline__ int32_t SweepMovingTargets(const m3WorldView& w, const m
     return hits;
 }
 
+// The bounds of shape o's tree leaf as this step's broadphase left them:
+// its own copy, since the replay into the nodes runs beside the step (a
+// static body moved between steps moves its leaf like any other).  A world
+// that keeps no tree has no copy; its nodes stand still.
+__device__ __forceinline__ m3Aabb LeafBounds(const m3WorldView& w, const m3Scratch& s, int32_t o)
+{
+    if (w.sc->treeTracked != 0)
+    {
+        return s.leafBox[o];
+    }
+    const m3TreeNode& n = w.treeNodes[w.proxyId[o]];
+    m3Aabb leaf;
+    for (int32_t k = 0; k < 3; ++k)
+    {
+        leaf.lo[k] = n.lo[k];
+        leaf.hi[k] = n.hi[k];
+    }
+    return leaf;
+}
+
 // ---------------------------------------------------------------------
 // The tree arm of the continuous phase for one shape of a fast body
 // (solver.c:3081-3274): every static target whose tree leaf touches the
@@ -5095,10 +5115,9 @@ __device__ __noinline__ int32_t SweepMovingTargets(const m3WorldView& w, const m
 // Returns how many targets hit before `*fraction`; with exactly one,
 // `*fraction` becomes its fraction.  `*refusal` is set for a mesh or
 // voxel target.
-__device__ __noinline__ int32_t SweepStaticTargets(const m3WorldView& w, const m3Pos3* com0,
-                                                   const m3Quat* rot0, int32_t i, int32_t sh,
-                                                   const int32_t* targets, int32_t targetCount,
-                                                   const double* lo,
+__device__ __noinline__ int32_t SweepStaticTargets(const m3WorldView& w, const m3Scratch& s,
+                                                   int32_t i, int32_t sh, const int32_t* targets,
+                                                   int32_t targetCount, const double* lo,
                                                    const double* hi, const m3Pos3& base,
                                                    const m3ProxyDev& proxyB,
                                                    const m3SweepDev& fastSweep, m3real* fraction,
@@ -5130,7 +5149,7 @@ __device__ __noinline__ int32_t SweepStaticTargets(const m3WorldView& w, const m
         {
             continue;
         }
-        const m3TreeNode& leaf = w.treeNodes[w.proxyId[o]];
+        const m3Aabb leaf = LeafBounds(w, s, o);
         if (!(leaf.lo[0] <= hi[0] && lo[0] <= leaf.hi[0] && leaf.lo[1] <= hi[1] &&
               lo[1] <= leaf.hi[1] && leaf.lo[2] <= hi[2] && lo[2] <= leaf.hi[2]))
         {
@@ -5159,7 +5178,7 @@ __device__ __noinline__ int32_t SweepStaticTargets(const m3WorldView& w, const m
         proxyA.count = ProxyPoints(w, o, &proxyA.points, scratchA, &proxyA.radius);
         // The target's sweep relative to the fast body's base
         // (solver.c:3065-3079).
-        const m3Pos3 oc0 = com0[ob];
+        const m3Pos3 oc0 = s.com0[ob];
         const m3Transform oxf = w.xf[ob];
         const m3Vec3 orlc = m3RotateVec3(oxf.q, w.lc[ob]);
         m3SweepDev sweepA;
@@ -5169,7 +5188,7 @@ __device__ __noinline__ int32_t SweepStaticTargets(const m3WorldView& w, const m
         sweepA.c2 = v3((m3real)(oxf.p.x + (double)orlc.x - base.x),
                        (m3real)(oxf.p.y + (double)orlc.y - base.y),
                        (m3real)(oxf.p.z + (double)orlc.z - base.z));
-        sweepA.q1 = rot0[ob];
+        sweepA.q1 = s.rot0[ob];
         sweepA.q2 = oxf.q;
         int32_t state;
         const m3real t =
@@ -5371,9 +5390,9 @@ __global__ void __launch_bounds__(M3_BLOCK, 2) m3FinishKernel(const m3WorldView*
                     int32_t refusal = 0;
                     const m3real entry = fraction;
                     int32_t hits =
-                        staticTargets ? SweepStaticTargets(w, s.com0, s.rot0, i, sh, targets,
-                                                           targetCount, lo, hi, base, proxyB,
-                                                           fastSweep, &fraction, &refusal)
+                        staticTargets ? SweepStaticTargets(w, s, i, sh, targets, targetCount, lo, hi,
+                                                           base, proxyB, fastSweep, &fraction,
+                                                           &refusal)
                                       : 0;
                     if (pass == 1)
                     {
