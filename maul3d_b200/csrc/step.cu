@@ -5091,7 +5091,8 @@ __device__ __noinline__ int32_t SweepMovingTargets(const m3WorldView& w, const m
 // The bounds of shape o's tree leaf as this step's broadphase left them:
 // its own copy, since the replay into the nodes runs beside the step (a
 // static body moved between steps moves its leaf like any other).  A world
-// that keeps no tree has no copy; its nodes stand still.
+// that keeps no tree has no copy and its nodes stand still: a leaf that the
+// broadphase would have moved has the bounds it would have been given.
 __device__ __forceinline__ m3Aabb LeafBounds(const m3WorldView& w, const m3Scratch& s, int32_t o)
 {
     if (w.sc->treeTracked != 0)
@@ -5099,11 +5100,15 @@ __device__ __forceinline__ m3Aabb LeafBounds(const m3WorldView& w, const m3Scrat
         return s.leafBox[o];
     }
     const m3TreeNode& n = w.treeNodes[w.proxyId[o]];
+    const m3Aabb& b = s.aabb[o];
+    const bool kept = w.awake[w.shapeBody[o]] == 0 ||
+                      (n.lo[0] <= b.lo[0] && n.lo[1] <= b.lo[1] && n.lo[2] <= b.lo[2] &&
+                       b.hi[0] <= n.hi[0] && b.hi[1] <= n.hi[1] && b.hi[2] <= n.hi[2]);
     m3Aabb leaf;
     for (int32_t k = 0; k < 3; ++k)
     {
-        leaf.lo[k] = n.lo[k];
-        leaf.hi[k] = n.hi[k];
+        leaf.lo[k] = kept ? n.lo[k] : b.lo[k] - (double)M3_AABB_MARGIN;
+        leaf.hi[k] = kept ? n.hi[k] : b.hi[k] + (double)M3_AABB_MARGIN;
     }
     return leaf;
 }

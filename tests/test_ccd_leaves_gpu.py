@@ -5,8 +5,8 @@ A fast body is swept against the static shapes whose tree leaves touch its
 swept box (solver.c:3081-3274), the leaves as the step's own broadphase
 left them (broad_phase.c:516-538): a static box teleported into a ball's
 way must stop it in the very next step, in a world stepped alone, in a
-batch whose replays start after every step and in one whose replays
-gather.
+batch whose replays start after every step, in one whose replays gather,
+and in a served world, which keeps no tree.
 """
 import ctypes as C
 
@@ -77,3 +77,19 @@ def test_a_teleported_box_stops_the_ball_in_every_batch(m3, early):
     finally:
         for w in worlds + [alone]:
             w.destroy()
+
+
+def test_a_teleported_box_stops_the_ball_in_a_served_world(m3):
+    world, box = _world(m3)
+    _teleport(m3, box)
+    container = abi.encode_container(m3.lib, m3.snapshot(world), abi.journal_step(DT, 4))
+    server = m3.Server(device_budget=1 << 30, max_active=4)
+    try:
+        ticket = server.submit(container)
+        served, status = server.run()[ticket]
+        world.step(DT, 4, 1)
+        _stopped(world)
+        assert (served, status) == (world.hash(), 0)
+    finally:
+        server.close()
+        world.destroy()
