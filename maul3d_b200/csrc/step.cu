@@ -2366,6 +2366,24 @@ __device__ void ContinuousVersusPlane(const m3WorldView& w, int32_t body, int32_
 // share an SM (228 KB per SM, 1 KB reserved per block, static arrays).
 #define M3_TWO_BLOCK_SMEM (110 * 1024)
 
+// A kinematic body's velocities towards its target (solver.c:3945-3983).
+__device__ __forceinline__ void KinematicServo(const m3WorldView& w, int32_t i, float dt)
+{
+    const m3real servoInvDt = 1.0f / dt;
+    const m3Transform now = w.xf[i];
+    const m3Transform want = w.target[i];
+    w.v[i] = v3((m3real)(want.p.x - now.p.x) * servoInvDt,
+                (m3real)(want.p.y - now.p.y) * servoInvDt,
+                (m3real)(want.p.z - now.p.z) * servoInvDt);
+    m3Quat dq = m3MulQuat(want.q, q4(-now.q.x, -now.q.y, -now.q.z, now.q.w));
+    if (dq.w < 0.0f)
+    {
+        dq = q4(-dq.x, -dq.y, -dq.z, -dq.w);
+    }
+    w.w[i] = m3MulSV3(2.0f * servoInvDt, v3(dq.x, dq.y, dq.z));
+    w.hasTarget[i] = 0;
+}
+
 template <int NT, int MIN_BLOCKS>
 __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3PrepareKernel(const m3WorldView* views,
                                                             const int32_t* order, int32_t count,
@@ -3024,19 +3042,7 @@ __global__ void __launch_bounds__(NT, MIN_BLOCKS) m3PrepareKernel(const m3WorldV
             }
             if (type == M3_BODY_KINEMATIC && w.hasTarget[i] != 0)
             {
-                m3real servoInvDt = 1.0f / dt;
-                const m3Transform now = w.xf[i];
-                const m3Transform want = w.target[i];
-                w.v[i] = v3((m3real)(want.p.x - now.p.x) * servoInvDt,
-                            (m3real)(want.p.y - now.p.y) * servoInvDt,
-                            (m3real)(want.p.z - now.p.z) * servoInvDt);
-                m3Quat dq = m3MulQuat(want.q, q4(-now.q.x, -now.q.y, -now.q.z, now.q.w));
-                if (dq.w < 0.0f)
-                {
-                    dq = q4(-dq.x, -dq.y, -dq.z, -dq.w);
-                }
-                w.w[i] = m3MulSV3(2.0f * servoInvDt, v3(dq.x, dq.y, dq.z));
-                w.hasTarget[i] = 0;
+                KinematicServo(w, i, dt);
             }
         }
         s.moverFlag[i] = flag;
@@ -4210,7 +4216,9 @@ __global__ void __launch_bounds__(NT, 2) m3WidePrepareKernel(const m3WorldView* 
     M3_WIDE_MARK(M3_PHASE_COLOR)
 
     // Movers: alive, enabled, kinematic or awake dynamic, ascending
-    // (solver.c:3945-3983), with the kinematic servo.
+    // (solver.c:3945-3983).  The kinematic servo waits for the contact
+    // rows, which another kernel prepares from the velocities before it
+    // (m3WideSubstepKernel).
     for (int32_t i = gtid; i < bodyMax; i += gstride)
     {
         int32_t flag = 0;
@@ -4220,22 +4228,6 @@ __global__ void __launch_bounds__(NT, 2) m3WidePrepareKernel(const m3WorldView* 
             if (type == M3_BODY_KINEMATIC || (type == M3_BODY_DYNAMIC && w.awake[i] != 0))
             {
                 flag = 1;
-            }
-            if (type == M3_BODY_KINEMATIC && w.hasTarget[i] != 0)
-            {
-                m3real servoInvDt = 1.0f / dt;
-                const m3Transform now = w.xf[i];
-                const m3Transform want = w.target[i];
-                w.v[i] = v3((m3real)(want.p.x - now.p.x) * servoInvDt,
-                            (m3real)(want.p.y - now.p.y) * servoInvDt,
-                            (m3real)(want.p.z - now.p.z) * servoInvDt);
-                m3Quat dq = m3MulQuat(want.q, q4(-now.q.x, -now.q.y, -now.q.z, now.q.w));
-                if (dq.w < 0.0f)
-                {
-                    dq = q4(-dq.x, -dq.y, -dq.z, -dq.w);
-                }
-                w.w[i] = m3MulSV3(2.0f * servoInvDt, v3(dq.x, dq.y, dq.z));
-                w.hasTarget[i] = 0;
             }
         }
         s.moverFlag[i] = flag;
@@ -4384,6 +4376,17 @@ __global__ void __launch_bounds__(NT, 2) m3WideSubstepKernel(const m3WorldView* 
         }
         return true;
     };
+    // The kinematic servo (solver.c:3945-3983); a world with a kinematic
+    // mover runs its substeps here, and the loop's first barrier comes
+    // before anyone reads these velocities.
+    for (int32_t m = gtid; m < moverCount; m += gstride)
+    {
+        const int32_t i = s.movers[m];
+        if (w.btype[i] == M3_BODY_KINEMATIC && w.hasTarget[i] != 0)
+        {
+            KinematicServo(w, i, dt);
+        }
+    }
     // The substep loop (solver.c:4085-4203), unless m3IslandSubstepKernel
     // has run it.
     const int32_t loops = s.plan->islands != 0 ? 0 : substeps;
