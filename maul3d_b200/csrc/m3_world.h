@@ -163,11 +163,20 @@ struct m3StepProfile
 // table for the launch is free, else once M3_TREE_REPLAY_AT steps have
 // gathered, when the ring would overflow, or at once when something reads
 // or overwrites the tree.  A replay is a chain of its own and takes little
-// of a GPU that has room: eight steps of a 485-body world and its tree 10.3
-// -> 7.3 ms, of 64 worlds of up to 2,000 bodies 29.6 -> 23.1, of 2,048
-// worlds 98 -> 90 against gathering first.  4,096 worlds fill the GPU:
-// steps and trees together take as long either way (64 steps 386 -> 384
-// ms), and a step whose tree nobody reads yet 12.2 -> 15.2.
+// of a GPU that has room; in a batch that fills it, a replay beside the
+// steps moves time from the next reader into the steps.  Gathered against
+// early, ms for eight steps alone / with their trees:
+//   1,000 worlds of 32 to 2,048 bodies   50 / 80     against     69 / 70
+//   1,000 of 2,000                       86 / 124    against    116 / 116
+//   2,300 of 1,024                      104 / 144    against    138 / 138
+//   2,300 of 32 to 2,048                108 / 147    against    142 / 143
+//   2,300 of 12 (16 steps)               31 / 31     against     30 / 31
+//   4,096 of 32 to 2,048                189 / 252    against    247 / 248
+//   8,000 of 12 (16 steps)              108 / 110    against    109 / 111
+// Early is never longer with the trees.  In long runs (64 single steps) it
+// gains 15 % at 300 worlds of 500 bodies, 3 % at 1,000 of 2,000, 1 % at
+// 2,300 of 32 to 2,048 and nothing at 4,096, while steps whose trees nobody
+// reads yet are up to a third longer; the line lies where the gain ends.
 #define M3_TREE_LAG 32
 #define M3_TREE_REPLAY_AT 16
 #define M3_TREE_EARLY_WORLDS 16
